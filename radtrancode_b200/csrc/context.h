@@ -15,12 +15,12 @@
 #include "rtb_common.h"
 
 namespace rtb {
-int fwd_smem_bytes(int ng, int nsw, int ncol, int nlmax, int npath, int warps);
+int fwd_smem_bytes(int ng, int nsw, int nlmax, int npath, int warps);
 // warps per CTA a launch uses for a requested tile (tiles other than kWarps
 // exist for the usual instance only), and the blocks per SM it can hold
 int fwd_tile_warps(bool t2, bool ext, int warps);
 int fwd_blocks_per_sm(int smem, bool t2, bool ext, int warps, int ng);
-cudaError_t launch_fwd(const BatchDev& B, int nsw, int ncol, int nlmax, int npath, int grid, int warps,
+cudaError_t launch_fwd(const BatchDev& B, int nsw, int nlmax, int npath, int grid, int warps,
                        cudaStream_t st);
 
 // growable device buffer / pinned host buffer (grow-only, freed by release)
@@ -93,7 +93,7 @@ struct Staging {
     std::vector<float> ltemp;    // layer temperatures (K) of the spectra with air Rayleigh
     std::vector<int> nsub;       // device spectra (path groups) of each caller spectrum, in order
     std::vector<float> wfac;     // get_solar_wave at each wavenumber of iform 1 / 4 spectra
-    int Lmax = 0, nsw_max = 1, ncol_max = 1, nlmax_max = 1, npath_max = 1, ngas_max = 1;
+    int Lmax = 0, nsw_max = 1, nlmax_max = 1, npath_max = 1, ngas_max = 1;
     int64_t n_out = 0, n_jac = 0;
 };
 
@@ -178,7 +178,7 @@ struct rtb_context {
     int prepared = 0;
     int placed = 0;                       // outputs of the resident batch go to caller device arrays
     rtb::BatchDev B{};
-    int Lmax = 0, nsw_max = 1, ncol_max = 1, nlmax_max = 1, npath_max = 1, grid = 1;
+    int Lmax = 0, nsw_max = 1, nlmax_max = 1, npath_max = 1, grid = 1;
     std::vector<rtb::SpecDev> spec_host;
     std::vector<int> spec_npath, spec_nv, spec_nwave, spec_nlayer;
     int64_t n_out = 0, n_jac = 0;

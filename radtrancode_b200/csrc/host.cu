@@ -854,7 +854,6 @@ int pack_spectrum(rtb_context* c, const rtb_atm& a, Staging& st) {
     st.nsub.push_back(ngrp);
     st.Lmax = std::max(st.Lmax, a.nlayer);
     st.nsw_max = std::max(st.nsw_max, S.nsw);
-    st.ncol_max = std::max(st.ncol_max, S.ncol);
     st.nlmax_max = std::max(st.nlmax_max, nlmax);
     st.npath_max = std::max(st.npath_max, std::min(a.npath, kMaxPathDev));
     st.ngas_max = std::max(st.ngas_max, a.ngas);
@@ -912,7 +911,6 @@ void append_staging(Staging& dst, const Staging& src) {
     append_vec(dst.para_wave, src.para_wave);
     dst.Lmax = std::max(dst.Lmax, src.Lmax);
     dst.nsw_max = std::max(dst.nsw_max, src.nsw_max);
-    dst.ncol_max = std::max(dst.ncol_max, src.ncol_max);
     dst.nlmax_max = std::max(dst.nlmax_max, src.nlmax_max);
     dst.npath_max = std::max(dst.npath_max, src.npath_max);
     dst.ngas_max = std::max(dst.ngas_max, src.ngas_max);
@@ -1013,12 +1011,12 @@ int prepare_ex(rtb_context* c, int nspec, const rtb_atm* atms, const OutPlace* p
     const bool t2 = c->nt < 0, ext = st.any_para || st.any_ext;
     int bpsm_all = 0;
     for (int w : {2, 4, 8}) {
-        const int sm_w = fwd_smem_bytes(c->ng, st.nsw_max, st.ncol_max, st.nlmax_max, st.npath_max, w);
+        const int sm_w = fwd_smem_bytes(c->ng, st.nsw_max, st.nlmax_max, st.npath_max, w);
         c->bpsm_w[w] =
             (sm_w <= smem_max && fwd_tile_warps(t2, ext, w) == w) ? fwd_blocks_per_sm(sm_w, t2, ext, w, c->ng) : 0;
         bpsm_all = std::max(bpsm_all, c->bpsm_w[w]);
     }
-    const int smem = fwd_smem_bytes(c->ng, st.nsw_max, st.ncol_max, st.nlmax_max, st.npath_max, kWarps);
+    const int smem = fwd_smem_bytes(c->ng, st.nsw_max, st.nlmax_max, st.npath_max, kWarps);
     if (smem > smem_max)
         return fail(c, RTB_ERR_UNSUPPORTED, "spectrum needs %d B of shared memory (device %d)", smem, smem_max);
     if (c->bpsm_w[kWarps] <= 0) return fail(c, RTB_ERR_CUDA, "forward kernel cannot be resident (smem %d B)", smem);
@@ -1166,7 +1164,6 @@ int prepare_ex(rtb_context* c, int nspec, const rtb_atm* atms, const OutPlace* p
     B.cell_scratch = (float*)c->d_cells.p;
     c->Lmax = st.Lmax;
     c->nsw_max = st.nsw_max;
-    c->ncol_max = st.ncol_max;
     c->nlmax_max = st.nlmax_max;
     c->npath_max = st.npath_max;
     c->spec_host.clear();
@@ -1270,7 +1267,7 @@ int launch(rtb_context* c) {
             CUDA_TRY(c, cudaStreamBeginCapture(strm, cudaStreamCaptureModeRelaxed));
             cudaError_t e = cudaMemsetAsync(c->d_diag.p, 0, 64, strm);
             if (e == cudaSuccess)
-                e = launch_fwd(c->B, c->nsw_max, c->ncol_max, c->nlmax_max, c->npath_max, c->grid, c->tile_eff, strm);
+                e = launch_fwd(c->B, c->nsw_max, c->nlmax_max, c->npath_max, c->grid, c->tile_eff, strm);
             const cudaError_t e2 = cudaStreamEndCapture(strm, &g);
             if (e != cudaSuccess || e2 != cudaSuccess) {
                 if (g) cudaGraphDestroy(g);
@@ -1288,7 +1285,7 @@ int launch(rtb_context* c) {
     }
     CUDA_TRY(c, cudaMemsetAsync(c->d_diag.p, 0, 64, strm));
     CUDA_TRY(c, cudaEventRecord(c->ev0, strm));
-    CUDA_TRY(c, launch_fwd(c->B, c->nsw_max, c->ncol_max, c->nlmax_max, c->npath_max, c->grid, c->tile_eff, strm));
+    CUDA_TRY(c, launch_fwd(c->B, c->nsw_max, c->nlmax_max, c->npath_max, c->grid, c->tile_eff, strm));
     CUDA_TRY(c, cudaEventRecord(c->ev1, strm));
     c->launched_grid = c->grid;
     return RTB_OK;
@@ -1435,7 +1432,7 @@ int launch_static(rtb_context* c) {
     const cudaStream_t strm = stream_of(c);
     CUDA_TRY(c, cudaMemsetAsync(c->d_diag.p, 0, 64, strm));
     CUDA_TRY(c, cudaEventRecord(c->ev0, strm));
-    CUDA_TRY(c, launch_fwd(B, c->nsw_max, c->ncol_max, c->nlmax_max, c->npath_max, grid, c->tile_eff, strm));
+    CUDA_TRY(c, launch_fwd(B, c->nsw_max, c->nlmax_max, c->npath_max, grid, c->tile_eff, strm));
     CUDA_TRY(c, cudaEventRecord(c->ev1, strm));
     c->launched_grid = grid;
     return RTB_OK;

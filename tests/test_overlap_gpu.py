@@ -1,0 +1,60 @@
+"""The register sort of an overlap pass (csrc/overlap.cuh) on keys that its
+words, which leave out the keys' low bits, cannot order by themselves, and on
+keys already in order.  Integer results, so no tolerance: the sorted order of
+every pass that is not the reference heapsort's is the stable order of the
+mixed oracle, and bins and split positions are the oracle's in every pass."""
+import numpy as np
+import pytest
+
+from helpers import JAC_TOL, RAD_TOL, assignment, jac_err, rad_err
+from radtrancode_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _tables(kind, ng):
+    kt = synth.make_ktables([synth.CH4, synth.C2H6], np_=6, nt=5, ng=ng, vmin=600.0, delv=0.4, nbin=4, seed=ng)
+    a, b = kt.table(0), kt.table(1)
+    g = np.arange(ng, dtype=np.float64) / (ng - 1)
+    if kind == "flat":          # rows a few units in the last place apart, columns over many octaves
+        a[...] = (a[..., :1] * (1.0 + 4e-7 * np.arange(ng))).astype(np.float32)
+        b[...] = (b[..., :1] * 1e4 * 10.0 ** (9.0 * (g - 1.0))).astype(np.float32)
+    elif kind == "wide":        # keys over about a hundred octaves
+        a[...] = (a[..., :1] * 10.0 ** (28.0 * (g - 1.0))).astype(np.float32)
+        b[...] = (b[..., :1] * 10.0 ** (29.0 * (g - 1.0))).astype(np.float32)
+    elif kind == "apart":       # every row above the one before it: nothing to sort
+        a[...] = (a[..., :1] * 10.0 ** (0.2 * np.arange(ng))).astype(np.float32)
+        b[...] = (b[..., :1] * 1e-3 * (1.0 + g)).astype(np.float32)
+    return kt
+
+
+@pytest.mark.parametrize("kind", ["flat", "wide", "apart"])
+@pytest.mark.parametrize("ng", [3, 11, 12, 16, 17, 20, 22])
+def test_order_of_close_keys(ctx, oracle, kind, ng):
+    kt, cia = _tables(kind, ng), synth.make_cia(ng)
+    job = synth.make_job(kt, [synth.CH4, synth.C2H6], nlayer=13, seed=ng, nwave=4)
+    job.amount[:, 3] = job.amount[:, 2]            # both gases' columns alike
+    ctx.set_ktables(kt)
+    ctx.set_cia(cia)
+    ctx.set_debug(True)
+    try:
+        c, g, _ = ctx.cirsrtfg_wave(job)
+        perm, split = ctx.debug_bins(job)
+        st = ctx.stats()
+    finally:
+        ctx.set_debug(False)
+    _, (hperm, hsplit, _) = oracle.cirsrtfg_wave(kt, cia, job, oracle.ORC_MIXED, debug=True)
+    assert st["sort_passes"] == int((hperm[..., 0] >= 0).sum()) > 0
+    assert np.array_equal(split, hsplit)
+    assert np.array_equal(assignment(perm, split, ng), assignment(hperm, hsplit, ng))
+    oracle.lib().orc_set_sort_mode(1)
+    try:
+        _, (sperm, _, _) = oracle.cirsrtfg_wave(kt, cia, job, oracle.ORC_MIXED, debug=True)
+    finally:
+        oracle.lib().orc_set_sort_mode(0)
+    other = (perm != sperm).any(axis=-1)           # passes in another than the stable order
+    assert other.sum() <= st["exact_passes"]
+    assert np.array_equal(perm[other], hperm[other])
+    c64, g64, _ = oracle.cirsrtfg_wave(kt, cia, job, oracle.ORC_FP64)
+    assert rad_err(c, c64) <= RAD_TOL
+    assert jac_err(g, g64, job.nv) <= JAC_TOL
