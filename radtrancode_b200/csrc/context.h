@@ -15,12 +15,12 @@
 #include "rtb_common.h"
 
 namespace rtb {
-int fwd_smem_bytes(int ng, int nsw, int nlmax, int npath, int warps);
+int fwd_smem_bytes(int ng, int nsw, int ncol, int ngk, int nlmax, int npath, int warps);
 // warps per CTA a launch uses for a requested tile (tiles other than kWarps
 // exist for the usual instance only), and the blocks per SM it can hold
 int fwd_tile_warps(bool t2, bool ext, int warps);
 int fwd_blocks_per_sm(int smem, bool t2, bool ext, int warps, int ng);
-cudaError_t launch_fwd(const BatchDev& B, int nsw, int nlmax, int npath, int grid, int warps,
+cudaError_t launch_fwd(const BatchDev& B, int nsw, int ncol, int ngk, int nlmax, int npath, int grid, int warps,
                        cudaStream_t st);
 
 // growable device buffer / pinned host buffer (grow-only, freed by release)
@@ -93,7 +93,7 @@ struct Staging {
     std::vector<float> ltemp;    // layer temperatures (K) of the spectra with air Rayleigh
     std::vector<int> nsub;       // device spectra (path groups) of each caller spectrum, in order
     std::vector<float> wfac;     // get_solar_wave at each wavenumber of iform 1 / 4 spectra
-    int Lmax = 0, nsw_max = 1, nlmax_max = 1, npath_max = 1, ngas_max = 1;
+    int Lmax = 0, nsw_max = 1, ncol_max = 1, ngk_max = 1, nlmax_max = 1, npath_max = 1, ngas_max = 1;
     int64_t n_out = 0, n_jac = 0;
 };
 
@@ -151,7 +151,7 @@ struct rtb_context {
     std::vector<int64_t> tab_off;            // element offset of each table
     std::vector<float> vcen;                 // irregular grids: the first table's centres VCEN(NPOINT)
     std::vector<int> tab_id, tab_iso;        // the tables' gas and isotope ids (RTB_KTAB_BY_ID), empty: unknown
-    std::vector<std::vector<uint8_t>> nonzero;  // [tab][bin]: any value > 0 (get_kg.f:228-250)
+    std::vector<std::vector<uint8_t>> nonzero;  // [tab][bin]: bit 0 any value > 0 (get_kg.f:228-250), bit 1 kSliceLog
     rtb::DevBuf d_raw, d_log, d_delg, d_gord;
     // CIA
     int has_cia = 0;
@@ -178,7 +178,7 @@ struct rtb_context {
     int prepared = 0;
     int placed = 0;                       // outputs of the resident batch go to caller device arrays
     rtb::BatchDev B{};
-    int Lmax = 0, nsw_max = 1, nlmax_max = 1, npath_max = 1, grid = 1;
+    int Lmax = 0, nsw_max = 1, ncol_max = 1, ngk_max = 1, nlmax_max = 1, npath_max = 1, grid = 1;
     std::vector<rtb::SpecDev> spec_host;
     std::vector<int> spec_npath, spec_nv, spec_nwave, spec_nlayer;
     int64_t n_out = 0, n_jac = 0;

@@ -101,9 +101,9 @@ __host__ __device__ inline PathOff path_off(int nlmax, int ng, int nsw) {
 struct Layout {
     int warp_bytes, path_bytes, off_delg, off_region, total;
 };
-__host__ __device__ inline Layout make_layout(int ng, int nsw, int nlmax, int npath, int warps) {
+__host__ __device__ inline Layout make_layout(int ng, int nsw, int ncol, int ngk, int nlmax, int npath, int warps) {
     Layout Lo;
-    Lo.warp_bytes = align16(pass_scratch_bytes(ng));
+    Lo.warp_bytes = pass_scratch_bytes(ng, ncol, ngk);
     Lo.path_bytes = path_off(nlmax, ng, nsw).total;
     int o = 0;
     Lo.off_delg = o; o += 4 * kMaxNg;
@@ -115,9 +115,6 @@ __host__ __device__ inline Layout make_layout(int ng, int nsw, int nlmax, int np
     return Lo;
 }
 
-// ---------------------------------------------------------------------------
-// get_kg for one gas at one layer: lane g < ng returns k(g), dk/dT(g)
-// (get_kg.f:320-378 coincident branch, NaN -> 1e-37 at :443-471).
 // RANKK (radtran/cirsradg/rankk.f:34-117) on one thread: REAL cumulative
 // ordinates and distribution summed in the reference's order, the `<=` test,
 // the split fraction and the ig <= ng guards.  cont/dcont/weight are sorted
@@ -173,12 +170,24 @@ __device__ void rankk_lane(int ng, const float* gw, int nloop, float* cont, floa
     }
 }
 
+// a layer's place in the (P, T) grid of the tables, as get_kg takes it
+struct KgPos {
+    int ioff[4];
+    float u, v, dudt, u2, dudt2;
+};
+template <bool t2>
+__device__ __forceinline__ KgPos kg_pos(const LayerDev& L) {
+    const int4 o = __ldg((const int4*)L.ioff);
+    const float4 w = __ldg((const float4*)&L.u);
+    return KgPos{{o.x, o.y, o.z, o.w}, w.x, w.y, w.z, t2 ? L.u2 : 0.0f, t2 ? L.dudt2 : 0.0f};
+}
+
 // X and dX/dT of the four (P, T) corners of one g (get_kg.f:355-365 and
 // 413-423): bilinear in (ln p, T) for a table with one temperature grid; for
 // TEMP2 tables (NT < 0) linear in T along each pressure row with its own
 // weight, then linear in ln p
 template <bool t2>
-__device__ __forceinline__ void corners(const LayerDev& L, float Y1, float Y2, float Y3, float Y4, float& X,
+__device__ __forceinline__ void corners(const KgPos& L, float Y1, float Y2, float Y3, float Y4, float& X,
                                         float& DXDT) {
     const float U = L.u, V = L.v;
     const float a = __fsub_rn(1.0f, V), b = __fsub_rn(1.0f, U);
@@ -204,7 +213,7 @@ __device__ __forceinline__ void corners(const LayerDev& L, float Y1, float Y2, f
 // linear interpolation of one g of one table slice (no logarithms: the
 // non-coincident branch of get_kg.f:396-420)
 template <bool t2>
-__device__ __forceinline__ void interp_lin(const float* t, const LayerDev& L, int g, float& X, float& DXDT) {
+__device__ __forceinline__ void interp_lin(const float* t, const KgPos& L, int g, float& X, float& DXDT) {
     const float Y1 = __ldg(t + L.ioff[0] + g), Y2 = __ldg(t + L.ioff[1] + g);
     const float Y3 = __ldg(t + L.ioff[2] + g), Y4 = __ldg(t + L.ioff[3] + g);
     corners<t2>(L, Y1, Y2, Y3, Y4, X, DXDT);
@@ -215,7 +224,7 @@ __device__ __forceinline__ void interp_lin(const float* t, const LayerDev& L, in
 // rank-rebinned by rankk on lane 0.  scr: per-warp shared scratch of at least
 // 8 * kMaxNg floats + 2 * kMaxNg shorts.  Called by the whole warp.
 template <bool t2>
-__device__ void get_kg_lane_nc(const BatchDev& B, int64_t slice, float w1, float w2, const LayerDev& L, int lane,
+__device__ void get_kg_lane_nc(const BatchDev& B, int64_t slice, float w1, float w2, const KgPos& L, int lane,
                                float* scr,
                                float& k, float& dk) {
     const int ng = B.ng;
@@ -251,20 +260,21 @@ __device__ void get_kg_lane_nc(const BatchDev& B, int64_t slice, float w1, float
     __syncwarp();
 }
 
-template <bool t2, int NGC>
-__device__ __forceinline__ void get_kg_lane(const BatchDev& B, int64_t slice, const LayerDev& L, int lane,
-                                            float& k, float& dk) {
-    k = 0.0f;
-    dk = 0.0f;
-    if (slice < 0) return;
-    const float* raw = B.ktab_raw + slice;
-    const float y10 = __ldg(raw + L.ioff[0]), y20 = __ldg(raw + L.ioff[1]);
-    const float y30 = __ldg(raw + L.ioff[2]), y40 = __ldg(raw + L.ioff[3]);
-    const bool klog = !((y10 <= 0.0f) || (y20 <= 0.0f) || (y30 <= 0.0f) || (y40 <= 0.0f));
-    if (lane >= (NGC ? NGC : B.ng)) return;
-    const float* t = klog ? (B.ktab_log + slice) : raw;
-    const float Y1 = __ldg(t + L.ioff[0] + lane), Y2 = __ldg(t + L.ioff[1] + lane);
-    const float Y3 = __ldg(t + L.ioff[2] + lane), Y4 = __ldg(t + L.ioff[3] + lane);
+// get_kg for one g-ordinate of one gas at one layer (get_kg.f:320-378
+// coincident branch, NaN -> 1e-37 at :443-471)
+template <bool t2>
+__device__ __forceinline__ void get_kg_g(const BatchDev& B, int64_t slice, const KgPos& L, int g, float& k, float& dk) {
+    bool klog = (slice & kSliceLog) != 0;
+    slice &= ~kSliceLog;
+    if (!klog) {
+        const float* raw = B.ktab_raw + slice;
+        const float y10 = __ldg(raw + L.ioff[0]), y20 = __ldg(raw + L.ioff[1]);
+        const float y30 = __ldg(raw + L.ioff[2]), y40 = __ldg(raw + L.ioff[3]);
+        klog = !((y10 <= 0.0f) || (y20 <= 0.0f) || (y30 <= 0.0f) || (y40 <= 0.0f));
+    }
+    const float* t = (klog ? B.ktab_log : B.ktab_raw) + slice + g;
+    const float Y1 = __ldg(t + L.ioff[0]), Y2 = __ldg(t + L.ioff[1]);
+    const float Y3 = __ldg(t + L.ioff[2]), Y4 = __ldg(t + L.ioff[3]);
     float X, DXDT;
     corners<t2>(L, Y1, Y2, Y3, Y4, X, DXDT);
     if (klog) {
@@ -624,12 +634,12 @@ __device__ __forceinline__ void planck_fp32(int ispace, float vwave, float T, fl
 // fold), or 0 for an NG read at run time
 template <bool t2, bool ext, int WARPS, int NGC>
 __global__ void __launch_bounds__(WARPS * 32, 24 / WARPS)
-fwd_kernel(BatchDev B, int nsw_max, int nlmax_max, int npath_max) {
+fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, int npath_max) {
     constexpr int kThreads = WARPS * 32;
     constexpr int kWarps = WARPS;
     extern __shared__ __align__(16) char smem[];
     __shared__ SpecDev S_sh;
-    const Layout Lo = make_layout(B.ng, nsw_max, nlmax_max, npath_max, WARPS);
+    const Layout Lo = make_layout(B.ng, nsw_max, ncol_max, ngk_max, nlmax_max, npath_max, WARPS);
     const PathOff po = path_off(nlmax_max, B.ng, nsw_max);
     float* delg = (float*)(smem + Lo.off_delg);
     char* region = smem + Lo.off_region;
@@ -650,10 +660,14 @@ fwd_kernel(BatchDev B, int nsw_max, int nlmax_max, int npath_max) {
     ps.gd = (double*)wsm;
     ps.rec = (uint2*)(wsm + pass_rec_offset(ng));
     ps.word = (unsigned*)(wsm + pass_word_offset(ng));
-    ps.col = (float*)(wsm + pass_col_offset(ng));
+    ps.kg = (float2*)(wsm + pass_kg_offset(ng));
+    ps.col = (float*)(ps.kg + ngk_max * ng);
 
     __shared__ long long s_next;
     __shared__ int s_layer;
+    __shared__ int64_t s_slice[kMaxGasDev];
+    __shared__ unsigned char s_gas[kMaxGasDev];
+    __shared__ unsigned s_gmask;
     int64_t k_static = blockIdx.x;
     for (;;) {
         // next work item: grid-stride, or pulled from the launch's counter
@@ -689,6 +703,18 @@ fwd_kernel(BatchDev B, int nsw_max, int nlmax_max, int npath_max) {
         const WaveDev& W = B.wave[iw_glob];
         const int nsw = S.nsw, ncol = S.ncol;
 
+        // the gases with a table at this wavenumber
+        if (warp == 0) {
+            const int64_t sl = lane < S.ngas ? B.wg_slice[S.wg_off + (int64_t)iw * S.ngas + lane] : -1;
+            const unsigned m = __ballot_sync(kFull, sl >= 0);
+            if (sl >= 0) {
+                const int r = __popc(m & ((1u << lane) - 1u));
+                s_slice[r] = sl;
+                s_gas[r] = (unsigned char)lane;
+            }
+            if (lane == 0) s_gmask = m;
+        }
+        __syncthreads();
         // ---------------- stage A0: non-coincident gases -----------------
         // k-distributions of gases whose wavenumber falls between two table
         // points (rankk on lane 0), parked per (layer, gas) in the slot for
@@ -697,14 +723,14 @@ fwd_kernel(BatchDev B, int nsw_max, int nlmax_max, int npath_max) {
             const float* w2s = B.wg_w2 + S.wg_off + (int64_t)iw * S.ngas;
             const int64_t* slices = B.wg_slice + S.wg_off + (int64_t)iw * S.ngas;
             for (int l = warp; l < S.nlayer; l += kWarps) {
-                const LayerDev& L = B.lay[S.lay_off + l];
+                const KgPos L = kg_pos<t2>(B.lay[S.lay_off + l]);
                 float* ncw = tau_s + B.nc_off + ((int64_t)l * S.ngas) * kMaxNg * 2;
                 for (int g = 0; g < S.ngas; ++g)
                     if (w2s[g] >= 0.0f) {
                         float kv, dv;
                         const float w1 = B.wg_w1 ? B.wg_w1[S.wg_off + (int64_t)iw * S.ngas + g]
                                                  : __fsub_rn(1.0f, w2s[g]);
-                        get_kg_lane_nc<t2>(B, slices[g], w1, w2s[g], L, lane, (float*)wsm, kv, dv);
+                        get_kg_lane_nc<t2>(B, slices[g] < 0 ? -1 : slices[g] & ~kSliceLog, w1, w2s[g], L, lane, (float*)wsm, kv, dv);
                         if (lane < ng) {
                             ncw[(g * kMaxNg + lane) * 2] = kv;
                             ncw[(g * kMaxNg + lane) * 2 + 1] = dv;
@@ -725,21 +751,41 @@ fwd_kernel(BatchDev B, int nsw_max, int nlmax_max, int npath_max) {
             // addresses are formed where they are used: what lives across the
             // overlap passes costs registers, and those bound the resident warps
             auto amo = [&](int g) { return B.amo[S.lg_off + (int64_t)l * S.ngas + g]; };
-            auto get_kg = [&](int g, float& kv, float& dv) {
-                const int64_t at = S.wg_off + (int64_t)iw * S.ngas + g;
-                if (B.wg_w2 && B.wg_w2[at] >= 0.0f) {
-                    const float* ncw = tau_s + B.nc_off + ((int64_t)l * S.ngas + g) * kMaxNg * 2;
-                    kv = lane < ng ? ncw[lane * 2] : 0.0f;
-                    dv = lane < ng ? ncw[lane * 2 + 1] : 0.0f;
-                } else {
-                    get_kg_lane<t2, NGC>(B, B.wg_slice[at], B.lay[S.lay_off + l], lane, kv, dv);
+            // k and dk/dT of every gas with a table, (gas, g) spread over the lanes
+            {
+                const KgPos L = kg_pos<t2>(B.lay[S.lay_off + l]);
+                const int ntask = __popc(s_gmask) * ng;
+#pragma unroll 1
+                for (int t = lane; t < ntask; t += 32) {
+                    const int r = t / ng, g = t - r * ng;
+                    float kv, dv;
+                    const int64_t at = S.wg_off + (int64_t)iw * S.ngas + s_gas[r];
+                    if (B.wg_w2 && B.wg_w2[at] >= 0.0f) {
+                        const float* ncw = tau_s + B.nc_off + (((int64_t)l * S.ngas + s_gas[r]) * kMaxNg + g) * 2;
+                        kv = ncw[0];
+                        dv = ncw[1];
+                    } else {
+                        get_kg_g<t2>(B, s_slice[r], L, g, kv, dv);
+                    }
+                    ps.kg[t] = make_float2(kv, dv);
                 }
+                __syncwarp();
+            }
+            auto get_kg = [&](int g, float& kv, float& dv) {
+                const unsigned m = s_gmask;
+                float2 v = make_float2(0.0f, 0.0f);
+                if ((m >> g & 1u) && lane < ng) v = ps.kg[__popc(m & ((1u << g) - 1u)) * ng + lane];
+                kv = v.x;
+                dv = v.y;
             };
             // k(g) of the mix so far, its d/dT and its tracked gas columns (zero
             // until the gas is added), ordinate `lane` of each
             float kgv, cT;
-#pragma unroll
-            for (int c = 0; c < kMaxCols; ++c) ps.col[c * 32 + lane] = 0.0f;
+            auto zero_columns = [&]() {
+                if (lane < ng)
+                    for (int c = 0; c < ncol_max; ++c) ps.col[c * ng + lane] = 0.0f;
+            };
+            zero_columns();
             float k1v, d1v;
             get_kg(0, k1v, d1v);
             const float a1 = amo(0);
@@ -747,7 +793,7 @@ fwd_kernel(BatchDev B, int nsw_max, int nlmax_max, int npath_max) {
             cT = __fmul_rn(d1v, a1);
             int nE = 0;                         // tracked gases added so far
             if (S.col_gas[0] == 0) {
-                ps.col[lane] = k1v;
+                if (lane < ng) ps.col[lane] = k1v;
                 nE = 1;
             }
             for (int ig = 1; ig < S.ngas; ++ig) {
@@ -758,8 +804,7 @@ fwd_kernel(BatchDev B, int nsw_max, int nlmax_max, int npath_max) {
                 const bool z2 = __shfl_sync(kFull, k2v, ng - 1) == 0.0f;
                 float cAdd;
                 if (z1) {                       // noverlapg.f:88-97 / :152-162
-#pragma unroll
-                    for (int c = 0; c < kMaxCols; ++c) ps.col[c * 32 + lane] = 0.0f;
+                    zero_columns();
                     cT = __fmul_rn(d2v, a2);
                     cAdd = k2v;
                     kgv = __fmul_rn(k2v, a2);
@@ -781,7 +826,7 @@ fwd_kernel(BatchDev B, int nsw_max, int nlmax_max, int npath_max) {
                 }
                 // the added gas's column, where it is tracked
                 if (nE < kMaxCols && S.col_gas[nE] == ig) {
-                    ps.col[nE * 32 + lane] = cAdd;
+                    if (lane < ng) ps.col[nE * ng + lane] = cAdd;
                     ++nE;
                 }
             }
@@ -793,7 +838,7 @@ fwd_kernel(BatchDev B, int nsw_max, int nlmax_max, int npath_max) {
             for (int s = 0; s < nsw; ++s) {
                 // the tracked columns are the first active parameters, gases then T
                 float v = __shfl_sync(kFull, dtc, s);
-                if (s < ncol) v = __fadd_rn(v, s == S.sw_T ? cT : __fmul_rn(ps.col[s * 32 + lane], 1.0e-20f));
+                if (s < ncol) v = __fadd_rn(v, s == S.sw_T ? cT : __fmul_rn(ps.col[s * ng + min(lane, ng - 1)], 1.0e-20f));
                 if (lane < ng) dtau_s[((size_t)l * nsw + s) * ng + lane] = v;
             }
             __syncwarp();
@@ -953,12 +998,12 @@ fwd_kernel(BatchDev B, int nsw_max, int nlmax_max, int npath_max) {
 }
 
 // host-side helpers exported to host.cu
-int fwd_smem_bytes(int ng, int nsw, int nlmax, int npath, int warps) {
-    return make_layout(ng, nsw, nlmax, npath, warps).total;
+int fwd_smem_bytes(int ng, int nsw, int ncol, int ngk, int nlmax, int npath, int warps) {
+    return make_layout(ng, nsw, ncol, ngk, nlmax, npath, warps).total;
 }
 
 namespace {
-using FwdKern = void (*)(BatchDev, int, int, int);
+using FwdKern = void (*)(BatchDev, int, int, int, int, int);
 // the instance of a launch: t2 and ext as the batch needs them; a tile other
 // than kWarps, and NG = 20 as a constant, exist for the usual instance only
 // (one temperature grid, no extended options)
@@ -989,14 +1034,14 @@ int fwd_blocks_per_sm(int smem, bool t2, bool ext, int warps, int ng) {
     return n;
 }
 
-cudaError_t launch_fwd(const BatchDev& B, int nsw, int nlmax, int npath, int grid, int warps,
+cudaError_t launch_fwd(const BatchDev& B, int nsw, int ncol, int ngk, int nlmax, int npath, int grid, int warps,
                        cudaStream_t st) {
     const int w = fwd_tile_warps(B.t2, B.ext, warps);
-    const int smem = fwd_smem_bytes(B.ng, nsw, nlmax, npath, w);
+    const int smem = fwd_smem_bytes(B.ng, nsw, ncol, ngk, nlmax, npath, w);
     const FwdKern kern = fwd_instance(B.t2, B.ext, w, B.ng);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    kern<<<grid, w * 32, smem, st>>>(B, nsw, nlmax, npath);
+    kern<<<grid, w * 32, smem, st>>>(B, nsw, ncol, ngk, nlmax, npath);
     return cudaGetLastError();
 }
 

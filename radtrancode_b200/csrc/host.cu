@@ -689,7 +689,8 @@ int pack_spectrum(rtb_context* c, const rtb_atm& a, Staging& st) {
                 }
                 const int need = coinc ? n1 : n1 + 1;
                 if (need >= c->nbin[itab]) return fail(c, RTB_ERR_RANGE, "k-table %d has no record %d", itab, need);
-                if (c->nonzero[itab][n1]) slice = c->tab_off[itab] + (int64_t)n1 * np * std::abs(nt) * ng;
+                if (c->nonzero[itab][n1] & 1)
+                    slice = (c->tab_off[itab] + (int64_t)n1 * np * std::abs(nt) * ng) | (c->nonzero[itab][n1] & 2 ? kSliceLog : 0);
             } else if (itab >= 0) {
                 const float vmin = c->vmin[itab], delv = c->delv[itab];
                 float eps;
@@ -708,8 +709,8 @@ int pack_spectrum(rtb_context* c, const rtb_atm& a, Staging& st) {
                 const int need = coinc ? n1 : n1 + 1;
                 if (n1 < 0 || need >= c->nbin[itab])
                     return fail(c, RTB_ERR_RANGE, "wavenumber %g outside k-table %d", vwave, itab);
-                if (c->nonzero[itab][n1])
-                    slice = c->tab_off[itab] + (int64_t)n1 * np * std::abs(nt) * ng;
+                if (c->nonzero[itab][n1] & 1)
+                    slice = (c->tab_off[itab] + (int64_t)n1 * np * std::abs(nt) * ng) | (c->nonzero[itab][n1] & 2 ? kSliceLog : 0);
             }
             st.wg_slice.push_back(slice);
             st.wg_w2.push_back(w2);
@@ -854,6 +855,10 @@ int pack_spectrum(rtb_context* c, const rtb_atm& a, Staging& st) {
     st.nsub.push_back(ngrp);
     st.Lmax = std::max(st.Lmax, a.nlayer);
     st.nsw_max = std::max(st.nsw_max, S.nsw);
+    st.ncol_max = std::max(st.ncol_max, S.ncol - (S.sw_T >= 0 ? 1 : 0));   // gas columns
+    int ngk = 0;
+    for (int k = 0; k < a.ngas; ++k) ngk += a.ktab[k] >= 0 || a.ktab[k] == RTB_KTAB_BY_ID;
+    st.ngk_max = std::max(st.ngk_max, ngk);
     st.nlmax_max = std::max(st.nlmax_max, nlmax);
     st.npath_max = std::max(st.npath_max, std::min(a.npath, kMaxPathDev));
     st.ngas_max = std::max(st.ngas_max, a.ngas);
@@ -911,6 +916,8 @@ void append_staging(Staging& dst, const Staging& src) {
     append_vec(dst.para_wave, src.para_wave);
     dst.Lmax = std::max(dst.Lmax, src.Lmax);
     dst.nsw_max = std::max(dst.nsw_max, src.nsw_max);
+    dst.ncol_max = std::max(dst.ncol_max, src.ncol_max);
+    dst.ngk_max = std::max(dst.ngk_max, src.ngk_max);
     dst.nlmax_max = std::max(dst.nlmax_max, src.nlmax_max);
     dst.npath_max = std::max(dst.npath_max, src.npath_max);
     dst.ngas_max = std::max(dst.ngas_max, src.ngas_max);
@@ -1011,12 +1018,12 @@ int prepare_ex(rtb_context* c, int nspec, const rtb_atm* atms, const OutPlace* p
     const bool t2 = c->nt < 0, ext = st.any_para || st.any_ext;
     int bpsm_all = 0;
     for (int w : {2, 4, 8}) {
-        const int sm_w = fwd_smem_bytes(c->ng, st.nsw_max, st.nlmax_max, st.npath_max, w);
+        const int sm_w = fwd_smem_bytes(c->ng, st.nsw_max, st.ncol_max, st.ngk_max, st.nlmax_max, st.npath_max, w);
         c->bpsm_w[w] =
             (sm_w <= smem_max && fwd_tile_warps(t2, ext, w) == w) ? fwd_blocks_per_sm(sm_w, t2, ext, w, c->ng) : 0;
         bpsm_all = std::max(bpsm_all, c->bpsm_w[w]);
     }
-    const int smem = fwd_smem_bytes(c->ng, st.nsw_max, st.nlmax_max, st.npath_max, kWarps);
+    const int smem = fwd_smem_bytes(c->ng, st.nsw_max, st.ncol_max, st.ngk_max, st.nlmax_max, st.npath_max, kWarps);
     if (smem > smem_max)
         return fail(c, RTB_ERR_UNSUPPORTED, "spectrum needs %d B of shared memory (device %d)", smem, smem_max);
     if (c->bpsm_w[kWarps] <= 0) return fail(c, RTB_ERR_CUDA, "forward kernel cannot be resident (smem %d B)", smem);
@@ -1164,6 +1171,8 @@ int prepare_ex(rtb_context* c, int nspec, const rtb_atm* atms, const OutPlace* p
     B.cell_scratch = (float*)c->d_cells.p;
     c->Lmax = st.Lmax;
     c->nsw_max = st.nsw_max;
+    c->ncol_max = st.ncol_max;
+    c->ngk_max = st.ngk_max;
     c->nlmax_max = st.nlmax_max;
     c->npath_max = st.npath_max;
     c->spec_host.clear();
@@ -1267,7 +1276,7 @@ int launch(rtb_context* c) {
             CUDA_TRY(c, cudaStreamBeginCapture(strm, cudaStreamCaptureModeRelaxed));
             cudaError_t e = cudaMemsetAsync(c->d_diag.p, 0, 64, strm);
             if (e == cudaSuccess)
-                e = launch_fwd(c->B, c->nsw_max, c->nlmax_max, c->npath_max, c->grid, c->tile_eff, strm);
+                e = launch_fwd(c->B, c->nsw_max, c->ncol_max, c->ngk_max, c->nlmax_max, c->npath_max, c->grid, c->tile_eff, strm);
             const cudaError_t e2 = cudaStreamEndCapture(strm, &g);
             if (e != cudaSuccess || e2 != cudaSuccess) {
                 if (g) cudaGraphDestroy(g);
@@ -1285,7 +1294,7 @@ int launch(rtb_context* c) {
     }
     CUDA_TRY(c, cudaMemsetAsync(c->d_diag.p, 0, 64, strm));
     CUDA_TRY(c, cudaEventRecord(c->ev0, strm));
-    CUDA_TRY(c, launch_fwd(c->B, c->nsw_max, c->nlmax_max, c->npath_max, c->grid, c->tile_eff, strm));
+    CUDA_TRY(c, launch_fwd(c->B, c->nsw_max, c->ncol_max, c->ngk_max, c->nlmax_max, c->npath_max, c->grid, c->tile_eff, strm));
     CUDA_TRY(c, cudaEventRecord(c->ev1, strm));
     c->launched_grid = c->grid;
     return RTB_OK;
@@ -1432,7 +1441,7 @@ int launch_static(rtb_context* c) {
     const cudaStream_t strm = stream_of(c);
     CUDA_TRY(c, cudaMemsetAsync(c->d_diag.p, 0, 64, strm));
     CUDA_TRY(c, cudaEventRecord(c->ev0, strm));
-    CUDA_TRY(c, launch_fwd(B, c->nsw_max, c->nlmax_max, c->npath_max, grid, c->tile_eff, strm));
+    CUDA_TRY(c, launch_fwd(B, c->nsw_max, c->ncol_max, c->ngk_max, c->nlmax_max, c->npath_max, grid, c->tile_eff, strm));
     CUDA_TRY(c, cudaEventRecord(c->ev1, strm));
     c->launched_grid = grid;
     return RTB_OK;
@@ -1580,7 +1589,9 @@ int rtb_set_ktables(rtb_context* c, int ntab, int np, int nt, int ng, const floa
             uint8_t any = 0;
             for (int64_t i = 0; i < slice; ++i)
                 if (s[i] > 0.0f) { any = 1; break; }
-            c->nonzero[t][b] = any;
+            bool log0 = true;
+            for (int64_t i = 0; i < slice; i += ng) log0 = log0 && !(s[i] <= 0.0f);
+            c->nonzero[t][b] = (uint8_t)(any | (log0 ? 2 : 0));
         }
     }
     for (int64_t i = 0; i < total; ++i) lg[i] = (float)std::log((double)data[i]);

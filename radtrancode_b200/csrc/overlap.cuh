@@ -138,18 +138,22 @@ __device__ __forceinline__ void warp_sort(float (&x)[E], int lane) {
 }
 
 // Scratch of one warp's pass, in sorted order: the elements' words, then their
-// records, and the FP64 prefix of the weights over each lane's chunk.  gd also
-// takes the heapsort's words.
+// records, and the FP64 prefix of the weights over each lane's chunk (the
+// positions from NG * NG on are pads).  gd also takes the heapsort's words.
 struct PassScratch {
-    double* gd;        // [NG * NG]
-    uint2* rec;        // [NG * NG + 1]: {key * weight, word}; the last one a pad
+    double* gd;        // [32 * chunk]
+    uint2* rec;        // [32 * chunk + 1]: {key * weight, word}; the last one an empty element
     unsigned* word;    // position p at p + (p >> 4): lanes writing E consecutive positions do not share a bank
-    float* col;        // [kMaxCols][32]: the mix's gas columns, ordinate g at lane g
+    float* col;        // [column][NG]: the mix's gas columns
+    float2* kg;        // [gas with a table][NG]: k and dk/dT of the layer's gases
 };
-__host__ __device__ constexpr int pass_rec_offset(int ng) { return (8 * ng * ng + 15) & ~15; }
-__host__ __device__ constexpr int pass_word_offset(int ng) { return pass_rec_offset(ng) + ((8 * (ng * ng + 1) + 15) & ~15); }
-__host__ __device__ constexpr int pass_col_offset(int ng) { return pass_word_offset(ng) + ((4 * (ng * ng + ng * ng / 16) + 15) & ~15); }
-__host__ __device__ constexpr int pass_scratch_bytes(int ng) { return pass_col_offset(ng) + 4 * 32 * kMaxCols; }
+__host__ __device__ constexpr int pass_chunk(int ng) { return (ng * ng + 31) / 32; }
+__host__ __device__ constexpr int pass_rec_offset(int ng) { return 8 * 32 * pass_chunk(ng); }
+__host__ __device__ constexpr int pass_word_offset(int ng) { return pass_rec_offset(ng) + 8 * (32 * pass_chunk(ng) + 2); }
+__host__ __device__ constexpr int pass_kg_offset(int ng) { return pass_word_offset(ng) + 4 * (34 * pass_chunk(ng) + 2); }
+__host__ __device__ constexpr int pass_scratch_bytes(int ng, int ncol, int ngk) {
+    return (pass_kg_offset(ng) + 8 * ngk * ng + 4 * ncol * ng + 15) & ~15;
+}
 
 template <int N>
 struct Const {              // a compile-time number as an argument
@@ -191,8 +195,8 @@ __device__ __forceinline__ void add_columns(ColSum<NE>& acc, unsigned w, float s
 // sum, and where that could move its REAL value (the sum within 2^-43 of a
 // rounding boundary) the running sum is formed as well.
 template <int NE>
-__device__ __forceinline__ void walk_bins(const PassScratch& ps, int ng, int nloop, int lane, int c_last, int sp, double frac, double gprev, double tot, float ws, unsigned word, float a,
-                                          float b, float dg, float uT, float vT, float vAdd, float& kg, float& cT,
+__device__ __forceinline__ void walk_bins(const PassScratch& ps, int ng, int nloop, int empty, int lane, int c_last, int sp, double frac, double gprev, double tot, float ws, unsigned word, float a,
+                                          float b, float dg, float uT, int nE, float vT, float vAdd, float& kg, float& cT,
                                           float& cAdd) {
     const bool opens = lane > 0 && lane < ng && lane <= c_last, closes = lane < c_last;
     // the split element of the boundary below the bin
@@ -205,7 +209,7 @@ __device__ __forceinline__ void walk_bins(const PassScratch& ps, int ng, int nlo
     const int cnt = in ? pend - p0 : 0;
     float uE[NE];
 #pragma unroll
-    for (int e = 0; e < NE; ++e) uE[e] = ps.col[e * 32 + lane];
+    for (int e = 0; e < NE; ++e) uE[e] = e < nE && lane < ng ? ps.col[e * ng + lane] : 0.0f;
     ColSum<NE> g;
     g.T = 0.0f;
     g.add = 0.0f;
@@ -221,7 +225,7 @@ __device__ __forceinline__ void walk_bins(const PassScratch& ps, int ng, int nlo
     const int nmax = __reduce_max_sync(kFull, cnt);
 #pragma unroll 1
     for (int k = 0; k < nmax; ++k) {
-        const uint2 r = ps.rec[k < cnt ? p0 + k : nloop];
+        const uint2 r = ps.rec[k < cnt ? p0 + k : empty];
         const float w = __fmul_rn(__shfl_sync(kFull, dg, r.y >> 5), __shfl_sync(kFull, dg, r.y));
         acc = __fadd_rn(acc, __uint_as_float(r.x));
         add_columns<NE>(g, r.y, w, uT, uE, vT, vAdd);
@@ -239,7 +243,7 @@ __device__ __forceinline__ void walk_bins(const PassScratch& ps, int ng, int nlo
         sum = first;
 #pragma unroll 1
         for (int k = 0; k < nmax; ++k) {
-            const unsigned q = ps.rec[k < cnt ? p0 + k : nloop].y;
+            const unsigned q = ps.rec[k < cnt ? p0 + k : empty].y;
             sum = __dadd_rn(sum, (double)__fmul_rn(__shfl_sync(kFull, dg, q >> 5), __shfl_sync(kFull, dg, q)));
         }
         sum = __dadd_rn(sum, last);
@@ -251,7 +255,8 @@ __device__ __forceinline__ void walk_bins(const PassScratch& ps, int ng, int nlo
     cT = g.T * inv;
     cAdd = g.add * inv;
 #pragma unroll
-    for (int e = 0; e < NE; ++e) ps.col[e * 32 + lane] = g.e[e] * inv;
+    for (int e = 0; e < NE; ++e)
+        if (e < nE && lane < ng) ps.col[e * ng + lane] = g.e[e] * inv;
 }
 
 // One overlap pass.  On entry lane g holds a = k1(g) [* a1], b = k2(g) * a2, the
@@ -302,13 +307,14 @@ __device__ __forceinline__ void sort_pass(const BatchDev& B, const PassScratch& 
         disjoint = disjoint && net;
         dgn.block_exact += disjoint;
     }
-    const int ch = (nloop + 31) >> 5;            // sorted positions a lane runs over below
-    const int c0 = min(lane * ch, nloop), c1 = min(c0 + ch, nloop);
+    const int ch = (nloop + 31) >> 5;            // sorted positions a lane runs over below, pads at the end
+    const int c0 = lane * ch;
+    if (lane >= ng) a = __int_as_float(0x7fffffff);   // a pad's key: NaN, neither below nor equal to any
     if (disjoint) {
 #pragma unroll 1
-        for (int p = lane; p < nloop; p += 32) {
+        for (int p = lane; p < 32 * ch; p += 32) {
             const int i = p / ng;
-            ps.word[p + (p >> 4)] = (unsigned)(i << 5 | (p - i * ng));
+            ps.word[p + (p >> 4)] = p < nloop ? (unsigned)(i << 5 | (p - i * ng)) : kIdMask;
         }
     } else if (net) {
         const unsigned mul = 1u << (kIdBits - sh), sub = smin * mul;
@@ -364,9 +370,9 @@ __device__ __forceinline__ void sort_pass(const BatchDev& B, const PassScratch& 
         if (lane == 0) heapsort_words(nloop, W);
         __syncwarp();
 #pragma unroll 1
-        for (int p = lane; p < nloop; p += 32) {
-            const int e = (int)(unsigned)W[p], i = e / ng;
-            ps.word[p + (p >> 4)] = (unsigned)(i << 5 | (e - i * ng));
+        for (int p = lane; p < 32 * ch; p += 32) {
+            const int e = p < nloop ? (int)(unsigned)W[p] : 0, i = e / ng;
+            ps.word[p + (p >> 4)] = p < nloop ? (unsigned)(i << 5 | (e - i * ng)) : kIdMask;
         }
         __syncwarp();
         exact = true;
@@ -392,31 +398,26 @@ __device__ __forceinline__ void sort_pass(const BatchDev& B, const PassScratch& 
             warp_sort<E, (NGC == 20 && E == 16) ? 4 : 1>(x, lane);
 #pragma unroll
             for (int t = 0; t < E; ++t)
-                if (lane * E + t < nloop) ps.word[lane * E + ((lane * E) >> 4) + t] = __float_as_uint(x[t]);
+                if (lane * E + t < 32 * ch) ps.word[lane * E + ((lane * E) >> 4) + t] = __float_as_uint(x[t]);
         }
         __syncwarp();
         double run = 0.0;
         bool wrong = false, tie = false;
-        const unsigned qprev = c0 > 0 && c0 < c1 ? ps.word[c0 - 1 + ((c0 - 1) >> 4)] : kIdMask;
+        const unsigned qprev = lane > 0 ? ps.word[c0 - 1 + ((c0 - 1) >> 4)] : kIdMask;   // lane 0: a pad
         float kprev = __fadd_rn(__shfl_sync(kFull, a, qprev >> 5), __shfl_sync(kFull, b, qprev));
-        if (lane == 0) kprev = __int_as_float(0x7fffffff);   // NaN: nothing comes before position 0
 #pragma unroll 1
-        for (int t = 0; t < ch; ++t) {
-            const int p = c0 + t;
-            const bool live = p < c1;
-            const unsigned q = live ? ps.word[p + (p >> 4)] : kIdMask;
+        for (int p = c0; p < c0 + ch; ++p) {
+            const unsigned q = ps.word[p + (p >> 4)];
             const float key = __fadd_rn(__shfl_sync(kFull, a, q >> 5), __shfl_sync(kFull, b, q));
             const float w = __fmul_rn(__shfl_sync(kFull, dg, q >> 5), __shfl_sync(kFull, dg, q));
             run = __dadd_rn(run, (double)w);
-            if (live) {
-                ps.gd[p] = run;
-                ps.rec[p] = make_uint2(__float_as_uint(__fmul_rn(key, w)), q);
-                wrong |= key < kprev;
-                tie |= key == kprev;
-            }
+            ps.gd[p] = run;
+            ps.rec[p] = make_uint2(__float_as_uint(__fmul_rn(key, w)), q);
+            wrong |= key < kprev;
+            tie |= key == kprev;
             kprev = key;
         }
-        if (lane == 0) ps.rec[nloop] = make_uint2(0u, kIdMask);
+        if (lane == 0) ps.rec[32 * ch] = make_uint2(0u, kIdMask);
         if (!exact && !disjoint && !again && __any_sync(kFull, wrong)) {
             // words anew: the first position of the element's group of equal
             // leading bits << sh | the bits left out so far
@@ -428,7 +429,7 @@ __device__ __forceinline__ void sort_pass(const BatchDev& B, const PassScratch& 
             };
             int first = 0;
 #pragma unroll 1
-            for (int p = c0; p < c1; ++p)
+            for (int p = c0; p < min(c0 + ch, nloop); ++p)
                 if (starts(p, ps.word[p + (p >> 4)])) first = p;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) first = max(first, __shfl_up_sync(kFull, first, o));
@@ -436,10 +437,9 @@ __device__ __forceinline__ void sort_pass(const BatchDev& B, const PassScratch& 
             __syncwarp();
             unsigned* nw = (unsigned*)ps.gd;
 #pragma unroll 1
-            for (int t = 0; t < ch; ++t) {
-                const int p = c0 + t;
-                const bool live = p < c1;
-                const unsigned q = live ? ps.word[p + (p >> 4)] : kIdMask;
+            for (int p = c0; p < c0 + ch; ++p) {
+                const bool live = p < nloop;
+                const unsigned q = ps.word[p + (p >> 4)];
                 const float key = __fadd_rn(__shfl_sync(kFull, a, q >> 5), __shfl_sync(kFull, b, q));
                 if (live) {
                     if (starts(p, q)) first = p;
@@ -473,11 +473,11 @@ __device__ __forceinline__ void sort_pass(const BatchDev& B, const PassScratch& 
         }
         tot = __shfl_sync(kFull, incl, 31);
         const double bL = __shfl_sync(kFull, base, L);
-        const int lo0 = min(L * ch, nloop);
+        const int lo0 = L * ch;
         const bool found = lane < ng && tot >= gb;
         sp = nloop;
         if (found) {
-            int lo = lo0, hi = min(lo0 + ch, nloop);
+            int lo = lo0, hi = lo0 + ch;
             while (lo < hi) {
                 const int mid = (lo + hi) >> 1;
                 if (__dadd_rn(ps.gd[mid], bL) >= gb) hi = mid; else lo = mid + 1;
@@ -532,7 +532,7 @@ __device__ __forceinline__ void sort_pass(const BatchDev& B, const PassScratch& 
         dgn.irregular += 1;
         float acc = 0.0f, nT = 0.0f, nA = 0.0f;
         float* nc = (float*)ps.gd;               // the gas columns' new values
-        for (int c = 0; c < nE; ++c) nc[c * 32 + lane] = 0.0f;
+        for (int c = 0; c < nE; ++c) nc[c * 32 + lane] = 0.0f;   // lanes' own entries
         int ig = 0;
         double sum = 0.0, gp = 0.0;
 #pragma unroll 1
@@ -562,7 +562,7 @@ __device__ __forceinline__ void sort_pass(const BatchDev& B, const PassScratch& 
                 if (lane == ig)
                     for (int c = 0; c < nE; ++c)
                         nc[c * 32 + lane] = __fadd_rn(nc[c * 32 + lane],
-                                                      __fmul_rn(__fmul_rn(share, ps.col[c * 32 + ((q >> 5) & 31)]), w));
+                                                      __fmul_rn(__fmul_rn(share, ps.col[c * ng + ((q >> 5) & 31)]), w));
                 if (part == 0) {
                     sum = closes ? __dadd_rn(sum, __dmul_rn(fr, (double)w)) : __dadd_rn(sum, (double)w);
                     if (!closes) break;
@@ -593,7 +593,8 @@ __device__ __forceinline__ void sort_pass(const BatchDev& B, const PassScratch& 
         uT = nT;
         cAdd = nA;
         __syncwarp();
-        for (int c = 0; c < nE; ++c) ps.col[c * 32 + lane] = nc[c * 32 + lane];
+        if (lane < ng)
+            for (int c = 0; c < nE; ++c) ps.col[c * ng + lane] = nc[c * 32 + lane];
         __syncwarp();
         return;
     }
@@ -602,8 +603,8 @@ __device__ __forceinline__ void sort_pass(const BatchDev& B, const PassScratch& 
     // specialised on the number of gas columns that are not zero before the pass
     float cT;
     auto walk = [&](auto n) {
-        walk_bins<decltype(n)::value>(ps, ng, nloop, lane, c_last, sp, frac, gprev, tot, ws, word, a, b, dg, uT, vT,
-                                         vAdd, kg, cT, cAdd);
+        walk_bins<decltype(n)::value>(ps, ng, nloop, 32 * ch, lane, c_last, sp, frac, gprev, tot, ws, word, a, b, dg, uT, nE,
+                                      vT, vAdd, kg, cT, cAdd);
     };
     if (nE <= 1) walk(Const<1>());
     else if (nE == 2) walk(Const<2>());

@@ -37,6 +37,11 @@ struct LayerDev {
     float u2, dudt2;      // NT < 0: the temperature weight at pressure cp + 1 (get_kg.f:157-165)
 };
 
+// flag in a table slice's offset (BatchDev::wg_slice): the record's first
+// ordinate is above zero at every (P, T), so get_kg interpolates ln k there
+// (get_kg.f:320-331 tests the four corners) and the raw values are not read
+constexpr int64_t kSliceLog = (int64_t)1 << 62;
+
 // per-wavenumber constants
 struct WaveDev {
     float vwave;          // calculation wavenumber
@@ -110,7 +115,7 @@ struct BatchDev {
     const LayerDev* lay;
     const float* amo;            // [.. nlayer][ngas] amount*1e-20
     const WaveDev* wave;
-    const int64_t* wg_slice;     // [.. nwave][ngas] element offset of the table slice, -1 = zero
+    const int64_t* wg_slice;     // [.. nwave][ngas] element offset of the table slice (| kSliceLog), -1 = zero
     const float* wg_w2;          // [.. nwave][ngas] non-coincident weight of slice+1 (< 0: coincident); may be null
     const float* wg_w1;          // [.. nwave][ngas] weight of slice (irregular grids); null: 1 - wg_w2
     const float* xsec;           // [.. nwave][ncont]
