@@ -99,7 +99,7 @@ __host__ __device__ inline PathOff path_off(int nlmax, int ng, int nsw) {
 }
 
 struct Layout {
-    int warp_bytes, path_bytes, off_delg, off_region, total;
+    int warp_bytes, path_bytes, off_delg, off_mtab, off_region, total;
 };
 __host__ __device__ inline Layout make_layout(int ng, int nsw, int ncol, int ngk, int nlmax, int npath, int warps) {
     Layout Lo;
@@ -108,6 +108,7 @@ __host__ __device__ inline Layout make_layout(int ng, int nsw, int ncol, int ngk
     int o = 0;
     Lo.off_delg = o; o += 4 * kMaxNg;
     o = align16(o);
+    Lo.off_mtab = o; o += (int)sizeof(MergeLane) * kMergeLevels * 32;
     Lo.off_region = o;
     const int a = warps * Lo.warp_bytes, b = npath * Lo.path_bytes;
     o += a > b ? a : b;
@@ -629,9 +630,10 @@ __device__ __forceinline__ void planck_fp32(int ispace, float vwave, float T, fl
 // item worked on at once -- the tile shape the autotuner chooses.  The
 // residency bound keeps 24 warps per SM at 80 registers: the passes wait on
 // shuffles and fixed-latency chains, and 16 warps at 128 registers took 4.28 ms
-// where 24 take 4.04 ms (120 layers, 4 absorbers, 2000 wavenumbers).  NGC: NG
-// as a compile-time constant (the overlap's sizes, offsets and loop bounds
-// fold), or 0 for an NG read at run time
+// where 24 take 4.04 ms (120 layers, 4 absorbers, 2000 wavenumbers).  NGC > 0:
+// NG as a compile-time constant (the overlap's sizes, offsets and loop bounds
+// fold); otherwise NG is read at run time, and -4 or -8 sort the elements of a
+// pass in that many registers per lane, 0 by merging rows
 template <bool t2, bool ext, int WARPS, int NGC>
 __global__ void __launch_bounds__(WARPS * 32, 24 / WARPS)
 fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, int npath_max) {
@@ -644,13 +646,16 @@ fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, in
     float* delg = (float*)(smem + Lo.off_delg);
     char* region = smem + Lo.off_region;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int ng = NGC ? NGC : B.ng;   // NGC > 0: the instance for NG = NGC (== B.ng)
+    constexpr int NG = NGC > 0 ? NGC : 0, E = NGC < 0 ? -NGC : 0;
+    const int ng = NG ? NG : B.ng;     // NGC > 0: the instance for NG = NGC (== B.ng)
     // per-CTA scratch slot in global memory (L2-resident): tau[l][g], dtau[l][s][g]
-    float* tau_s = B.cell_scratch + (int64_t)blockIdx.x * B.cell_slot;
-    float* dtau_s = tau_s + (int64_t)B.cell_Lmax * ng;
+    auto slot = [&]() { return B.cell_scratch + (int64_t)blockIdx.x * B.cell_slot; };
+    auto slot_dtau = [&]() { return slot() + (int64_t)B.cell_Lmax * ng; };
     for (int i = tid; i < ng; i += kThreads) delg[i] = B.delg[i];
     const float dg = lane < ng ? B.delg[lane] : 0.0f;                // this lane's g-ordinate weight
     const double gb = lane < ng ? B.g_ord[lane + 1] : 0.0;          // and upper bin boundary
+    MergeLane* mtab = (MergeLane*)(smem + Lo.off_mtab);
+    for (int i = tid; i < kMergeLevels * 32; i += kThreads) mtab[i] = merge_lane(ng, i / 32, i % 32);
     __shared__ unsigned long long s_count[5];
     if (tid < 5) s_count[tid] = 0;
     __syncthreads();
@@ -658,23 +663,23 @@ fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, in
     char* wsm = region + warp * Lo.warp_bytes;
     PassScratch ps;
     ps.gd = (double*)wsm;
-    ps.rec = (uint2*)(wsm + pass_rec_offset(ng));
-    ps.word = (unsigned*)(wsm + pass_word_offset(ng));
+    ps.rec = (uint2*)(wsm + pass_gd_bytes(ng));
+    ps.mtab = mtab;
     ps.kg = (float2*)(wsm + pass_kg_offset(ng));
     ps.col = (float*)(ps.kg + ngk_max * ng);
 
-    __shared__ long long s_next;
+    __shared__ int s_next;
     __shared__ int s_layer;
     __shared__ int64_t s_slice[kMaxGasDev];
     __shared__ unsigned char s_gas[kMaxGasDev];
     __shared__ unsigned s_gmask;
-    int64_t k_static = blockIdx.x;
+    int k_static = blockIdx.x;      // items are numbered in 32 bits (item_order)
     for (;;) {
         // next work item: grid-stride, or pulled from the launch's counter
         // (dynamic schedule); item_order maps the issue order to items
-        int64_t k;
+        int k;
         if (B.work_next) {
-            if (tid == 0) s_next = (long long)atomicAdd(B.work_next, 1ull);
+            if (tid == 0) s_next = (int)atomicAdd(B.work_next, 1ull);
             __syncthreads();
             k = s_next;
         } else {
@@ -682,7 +687,7 @@ fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, in
             k_static += gridDim.x;
         }
         if (k >= B.nitems) break;
-        const int64_t item = B.item_order ? (int64_t)B.item_order[k] : k;
+        const int item = B.item_order ? B.item_order[k] : k;
         // locate the spectrum of this item
         int lo = 0, hi = B.nspec - 1;
         while (lo < hi) {
@@ -699,9 +704,6 @@ fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, in
         __syncthreads();
         const SpecDev& S = S_sh;
         const int iw = (int)(item - B.item_start[sidx]);
-        const int64_t iw_glob = S.wave_off + iw;
-        const WaveDev& W = B.wave[iw_glob];
-        const int nsw = S.nsw, ncol = S.ncol;
 
         // the gases with a table at this wavenumber
         if (warp == 0) {
@@ -724,7 +726,7 @@ fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, in
             const int64_t* slices = B.wg_slice + S.wg_off + (int64_t)iw * S.ngas;
             for (int l = warp; l < S.nlayer; l += kWarps) {
                 const KgPos L = kg_pos<t2>(B.lay[S.lay_off + l]);
-                float* ncw = tau_s + B.nc_off + ((int64_t)l * S.ngas) * kMaxNg * 2;
+                float* ncw = slot() + B.nc_off + ((int64_t)l * S.ngas) * kMaxNg * 2;
                 for (int g = 0; g < S.ngas; ++g)
                     if (w2s[g] >= 0.0f) {
                         float kv, dv;
@@ -761,7 +763,7 @@ fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, in
                     float kv, dv;
                     const int64_t at = S.wg_off + (int64_t)iw * S.ngas + s_gas[r];
                     if (B.wg_w2 && B.wg_w2[at] >= 0.0f) {
-                        const float* ncw = tau_s + B.nc_off + (((int64_t)l * S.ngas + s_gas[r]) * kMaxNg + g) * 2;
+                        const float* ncw = slot() + B.nc_off + (((int64_t)l * S.ngas + s_gas[r]) * kMaxNg + g) * 2;
                         kv = ncw[0];
                         dv = ncw[1];
                     } else {
@@ -816,13 +818,7 @@ fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, in
                     mono = __all_sync(kFull, mono && (lane + 1 >= ng || k2v <= kn));
                     const float b = __fmul_rn(k2v, a2), vT = __fmul_rn(d2v, a2);
                     const int dbg_rec = B.dbg_perm && sidx == 0 ? (iw * S.nlayer + l) * (S.ngas - 1) + (ig - 1) : -1;
-                    auto pass = [&](auto e) {
-                        sort_pass<decltype(e)::value, NGC>(B, ps, ng, mono, kgv, b, dg, gb, cT, nE, vT, k2v, kgv, cAdd, lane,
-                                                           dgn, dbg_rec);
-                    };
-                    if (NGC ? NGC * NGC <= 128 : ng * ng <= 128) pass(Const<4>());
-                    else if (NGC ? NGC * NGC <= 256 : ng * ng <= 256) pass(Const<8>());
-                    else pass(Const<16>());
+                    sort_pass<E, NG>(B, ps, ng, mono, kgv, b, dg, gb, cT, nE, vT, k2v, kgv, cAdd, lane, dgn, dbg_rec);
                 }
                 // the added gas's column, where it is tracked
                 if (nE < kMaxCols && S.col_gas[nE] == ig) {
@@ -831,15 +827,17 @@ fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, in
                 }
             }
             // tau and dtau/dq per g (cirsradg_wave.f:744-790)
-            const int64_t il_glob = S.lay_off + l;
+            const int64_t il_glob = S.lay_off + l, iw_glob = S.wave_off + iw;
             float dtc;
-            const float taucon = continuum<ext>(B, S, B.lay[il_glob], W, iw_glob, il_glob, lane, dtc);
-            if (lane < ng) tau_s[l * ng + lane] = __fadd_rn(taucon, kgv);
-            for (int s = 0; s < nsw; ++s) {
+            const float taucon = continuum<ext>(B, S, B.lay[il_glob], B.wave[iw_glob], iw_glob, il_glob, lane, dtc);
+            float* tau_l = slot() + l * ng;
+            float* dtau_l = slot_dtau() + (size_t)l * S.nsw * ng;
+            if (lane < ng) tau_l[lane] = __fadd_rn(taucon, kgv);
+            for (int s = 0; s < S.nsw; ++s) {
                 // the tracked columns are the first active parameters, gases then T
                 float v = __shfl_sync(kFull, dtc, s);
-                if (s < ncol) v = __fadd_rn(v, s == S.sw_T ? cT : __fmul_rn(ps.col[s * ng + min(lane, ng - 1)], 1.0e-20f));
-                if (lane < ng) dtau_s[((size_t)l * nsw + s) * ng + lane] = v;
+                if (s < S.ncol) v = __fadd_rn(v, s == S.sw_T ? cT : __fmul_rn(ps.col[s * ng + min(lane, ng - 1)], 1.0e-20f));
+                if (lane < ng) dtau_l[s * ng + lane] = v;
             }
             __syncwarp();
         }
@@ -853,6 +851,10 @@ fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, in
         __syncthreads();
 
         // ---------------- stage B: paths ---------------------------------
+        const WaveDev& W = B.wave[S.wave_off + iw];
+        const float* tau_s = slot();
+        const float* dtau_s = slot_dtau();
+        const int nsw = S.nsw;
         for (int p = warp; p < S.npath; p += kWarps) {
             char* ps = region + p * Lo.path_bytes;
             float* drdt = (float*)(ps + po.drdt);
@@ -1006,17 +1008,25 @@ namespace {
 using FwdKern = void (*)(BatchDev, int, int, int, int, int);
 // the instance of a launch: t2 and ext as the batch needs them; a tile other
 // than kWarps, and NG = 20 as a constant, exist for the usual instance only
-// (one temperature grid, no extended options)
+// (one temperature grid, no extended options).  Up to 256 elements a pass are
+// sorted in registers, more are merged in shared memory: one spectrum of
+// 16-point tables (80 layers, 150 wavenumbers, 2 absorbers) takes 0.22 ms by
+// the first and 0.27 ms by the second, one of 20-point tables (120 layers, 2000
+// wavenumbers, 4 absorbers) 3.68 and 3.45 ms.
 constexpr int kNgConst = 20;
+template <bool t2, bool ext, int WARPS>
+FwdKern fwd_by_ng(int ng) {
+    if (!t2 && !ext && ng == kNgConst) return fwd_kernel<t2, ext, WARPS, t2 || ext ? 0 : kNgConst>;
+    if (ng * ng > 256) return fwd_kernel<t2, ext, WARPS, 0>;
+    if (ng * ng > 128) return fwd_kernel<t2, ext, WARPS, -8>;
+    return fwd_kernel<t2, ext, WARPS, -4>;
+}
 FwdKern fwd_instance(bool t2, bool ext, int warps, int ng) {
-    if (ext) return t2 ? fwd_kernel<true, true, kWarps, 0> : fwd_kernel<false, true, kWarps, 0>;
-    if (t2) return fwd_kernel<true, false, kWarps, 0>;
-    const bool c20 = ng == kNgConst;
-    switch (warps) {
-    case 2: return c20 ? fwd_kernel<false, false, 2, kNgConst> : fwd_kernel<false, false, 2, 0>;
-    case 8: return c20 ? fwd_kernel<false, false, 8, kNgConst> : fwd_kernel<false, false, 8, 0>;
-    default: return c20 ? fwd_kernel<false, false, kWarps, kNgConst> : fwd_kernel<false, false, kWarps, 0>;
-    }
+    if (ext) return t2 ? fwd_by_ng<true, true, kWarps>(ng) : fwd_by_ng<false, true, kWarps>(ng);
+    if (t2) return fwd_by_ng<true, false, kWarps>(ng);
+    if (warps == 2) return fwd_by_ng<false, false, 2>(ng);
+    if (warps == 8) return fwd_by_ng<false, false, 8>(ng);
+    return fwd_by_ng<false, false, kWarps>(ng);
 }
 }  // namespace
 

@@ -1,17 +1,19 @@
 // overlap.cuh -- one random-overlap pass of two k-distributions on one warp
 // (radtran/cirsradg/noverlapg.f:110-147, 175-190 with rankg.f:59-152).
 //
-// Lane g holds ordinate g of both distributions.  The NG*NG combined keys
-// A(i) + B(j) are sorted in registers, E consecutive positions of the sorted
-// order per lane, by a bitonic network; the cumulative weights come from a
-// warp scan, and lane b then walks bin b in the sorted order.
+// Lane g holds ordinate g of both distributions.  An element of the combined
+// distribution travels as one 32-bit word; the words are sorted in registers
+// (up to 256 elements) or by merging the NG rows of keys A(i) + B(j), which are
+// in order when B is monotone, in shared memory.  The cumulative weights come
+// from a warp scan, and lane b then walks bin b in the sorted order.
 //
-// What bounds it: instruction issue (2.4 of 4 per cycle and SM) and the
-// half-rate ALU pipe.  At 120 layers, 4 absorbers and 2000 wavenumbers (720000
-// passes of 400 keys, a third of them with nothing to sort) the forward kernel
-// takes 3.9 ms; with the 64-bit words of the keys merged row by row in shared
-// memory (800 cycles and 585 bank conflicts a pass and SM, against 540 cycles
-// and no shared memory for this sort) it took 5.45 ms.
+// What bounds it: instruction issue (2.5 of 4 per cycle and SM with 24 warps) and
+// the latency of shared memory and shuffles.  120 layers, 4 absorbers, 2000
+// wavenumbers (720000 passes of 400 keys, a third of them with rows already in
+// order): the forward kernel takes 3.41 ms, 3250 warp instructions a pass.  With
+// the merge on 64-bit words of key and element, and weights and columns in
+// shared-memory tables, it took 5.45 ms (4575 instructions and 585 bank
+// conflicts a pass); with the 400 words sorted in 16 registers a lane 3.68 ms.
 #pragma once
 #include <stdint.h>
 
@@ -22,13 +24,14 @@ namespace rtb {
 constexpr unsigned kFull = 0xffffffffu;
 
 // An element (i, j) of a pass in one 32-bit word: i << 5 | j in the low ten
-// bits, above them the leading bits of key - smallest key.  Words are compared
-// as positive floats, so they stay below the pattern of infinity; a pad word
-// lies above every element's and names the lanes (20, 20)..(31, 31) or
-// beyond NG, whose weight is zero.
+// bits, above them the leading bits of key - smallest key.  kEnd lies above
+// every word of the merge; the register sort compares words as positive floats,
+// with kPad above them all.  The element kIdMask names lane 31, whose weight is
+// zero.
 constexpr unsigned kIdBits = 10;
 constexpr unsigned kIdMask = (1u << kIdBits) - 1;
-constexpr unsigned kPadWord = 0x7f7ffc00u;
+constexpr unsigned kEnd = 0xffffffffu;
+constexpr unsigned kPad = 0x7f7fffffu;      // the largest finite float
 
 __device__ __forceinline__ float wkey(unsigned long long w) { return __uint_as_float((unsigned)(w >> 32)); }
 
@@ -84,6 +87,106 @@ __device__ __noinline__ void heapsort_words(int n, unsigned long long* W0) {
     }
 }
 
+constexpr int kMergeLevels = 5;   // merge levels of NG <= 32 rows
+
+// What a lane does at one merge level, for NG rows (run = NG << level).  Pair p
+// of runs (start st_p of n = NG^2) is served by lanes [L_p, L_p+1), L_p =
+// floor(32 st_p / n), which split it evenly: no lane's output range crosses a
+// pair, so every lane runs a single merge per level (14 steps for NG = 20).
+// Byte offsets: a and b the pair's runs in the source (b the kEnd after a where
+// there is no right run), diag of the range's first position in the pair, out
+// the range in the target; [lo, hi] what the bisection for the left run's share
+// starts from; len words.
+struct MergeLane {
+    unsigned short a, b, diag, lo, hi, out, len, pad;
+};
+__device__ inline MergeLane merge_lane(int ng, int level, int l) {
+    const int n = ng * ng, run = ng << level;
+    MergeLane M = {0, 0, 0, 0, 0, 0, 0, 0};
+    if (run >= n) return M;
+    const int two = run << 1, npairs = (n + two - 1) / two;
+    auto start = [&](int q) {                  // first output position of lane q
+        if (q >= 32) return n;
+        int p = 0;
+        while (p + 1 < npairs && (32 * (p + 1) * two) / n <= q) ++p;
+        const int st = p * two, sz = min(two, n - st);
+        const int lp = (32 * st) / n, lq = p + 1 < npairs ? (32 * (p + 1) * two) / n : 32;
+        return st + ((q - lp) * sz) / (lq - lp);
+    };
+    const int s = start(l), e = start(l + 1), p = s / two, ms = p * two;
+    if (s >= e) return M;
+    const int m = min(run, n - ms), ny = max(0, min(run, n - ms - run)), kk = s - ms;
+    M.a = (unsigned short)(4 * (2 * p * (run + 1)));
+    M.b = (unsigned short)(M.a + 4 * (ny > 0 ? run + 1 : m));
+    M.diag = (unsigned short)(4 * kk);
+    M.lo = (unsigned short)(4 * max(0, kk - ny));
+    M.hi = (unsigned short)(4 * min(kk, m));
+    M.out = (unsigned short)(two >= n ? 8 * s + 4 : 4 * (p * (two + 1) + kk));
+    M.len = (unsigned short)(e - s);
+    return M;
+}
+
+__device__ __forceinline__ unsigned lds32(unsigned at) {
+    unsigned v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(at) : "memory");
+    return v;
+}
+
+// One step of a merge on shared-memory byte addresses: the smaller of the two
+// front words to `out`, the next word of its run in its place.  Words differ,
+// and the kEnd after a run is never written out while the other run has words.
+__device__ __forceinline__ void merge_step(unsigned& x, unsigned& y, unsigned& pa, unsigned& pb, unsigned out) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .u32 o;\n\t"
+        "setp.lt.u32 p, %0, %1;\n\t"
+        "min.u32 o, %0, %1;\n\t"
+        "@p add.u32 %2, %2, 4;\n\t"
+        "@!p add.u32 %3, %3, 4;\n\t"
+        "st.shared.u32 [%4], o;\n\t"
+        "@p ld.shared.u32 %0, [%2];\n\t"
+        "@!p ld.shared.u32 %1, [%3];\n\t}"
+        : "+r"(x), "+r"(y), "+r"(pa), "+r"(pb)
+        : "r"(out)
+        : "memory");
+}
+
+// Sorts ng sorted rows of ng words, row i at i (ng + 1) with kEnd after it in
+// the buffer `from`, through `gd` and `rec` in turn; the last level reads gd and
+// writes the words of the records (rec[p].y, position p).  A level merges pairs
+// of runs of length run into runs of 2 run, each followed by kEnd: every lane
+// finds by bisection where its output range (mtab) starts in the pair's two
+// runs and merges from there.  Shared-memory byte addresses.
+template <int NGC>
+__device__ __forceinline__ void merge_rows(unsigned gd, unsigned rec, const MergeLane* mtab, int ng_run, int levels, int lane) {
+    const int ng = NGC ? NGC : ng_run, n = ng * ng;
+    unsigned from = (levels & 1) ? gd : rec;
+#pragma unroll 1
+    for (int level = 0; level < levels; ++level) {
+        const uint4 d = *(const uint4*)(mtab + level * 32 + lane);
+        const unsigned A = from + (d.x & 0xffffu), Bv = from + (d.x >> 16) + (d.y & 0xffffu);
+        unsigned lo = d.y >> 16, hi = d.z & 0xffffu;
+        while (lo < hi) {
+            const unsigned mid = ((lo + hi) >> 1) & ~3u;
+            if (lds32(A + mid) < lds32(Bv - 4 - mid)) lo = mid + 4; else hi = mid;
+        }
+        unsigned pa = A + lo, pb = Bv - lo;
+        unsigned x = lds32(pa), y = lds32(pb);
+        const bool last = level + 1 == levels;
+        const unsigned to = gd + rec - from, step = last ? 8u : 4u;
+        unsigned out = to + (d.z >> 16);
+        const unsigned end = out + step * (d.w & 0xffffu);
+#pragma unroll 2
+        for (; out < end; out += step) merge_step(x, y, pa, pb, out);
+        const int two = ng << (level + 1);
+        if (!last && lane * two < n) {
+            const unsigned at = to + 4 * (lane * (two + 1) + min(two, n - lane * two));
+            asm volatile("st.shared.u32 [%0], %1;" ::"r"(at), "r"(kEnd) : "memory");
+        }
+        __syncwarp();
+        from = to;
+    }
+}
+
 __device__ __forceinline__ void order(float& a, float& b) {
     const float lo = fminf(a, b);
     b = fmaxf(a, b);
@@ -91,16 +194,15 @@ __device__ __forceinline__ void order(float& a, float& b) {
 }
 
 // Sorts the 32 * E words of a warp (positive finite floats) ascending over
-// (lane, register).  Each lane's words are sorted first: by Batcher's network,
-// of which runs of P0 words that are already in order skip the first steps;
-// then bitonic merges over 2, 4, .. 32 lanes.  A lane that keeps the larger
+// (lane, register).  Each lane's words are sorted first by Batcher's network,
+// then by bitonic merges over 2, 4, .. 32 lanes.  A lane that keeps the larger
 // word of an exchange holds its words negated during it, so that every
 // exchange is one minimum with the negated partner: the sign changes run on
 // the FMA pipe, the minima on the half-rate ALU pipe, which bounds the sort.
-template <int E, int P0>
+template <int E>
 __device__ __forceinline__ void warp_sort(float (&x)[E], int lane) {
 #pragma unroll
-    for (int p = P0; p < E; p <<= 1)
+    for (int p = 1; p < E; p <<= 1)
 #pragma unroll
         for (int k = p; k >= 1; k >>= 1)
 #pragma unroll
@@ -137,20 +239,22 @@ __device__ __forceinline__ void warp_sort(float (&x)[E], int lane) {
     }
 }
 
-// Scratch of one warp's pass, in sorted order: the elements' words, then their
-// records, and the FP64 prefix of the weights over each lane's chunk (the
-// positions from NG * NG on are pads).  gd also takes the heapsort's words.
+// Scratch of one warp's pass, in sorted order: the elements' records and the
+// FP64 prefix of the weights over each lane's chunk (the positions from NG * NG
+// on are pads).  Both also take the merge's runs, and gd the heapsort's words.
 struct PassScratch {
     double* gd;        // [32 * chunk]
     uint2* rec;        // [32 * chunk + 1]: {key * weight, word}; the last one an empty element
-    unsigned* word;    // position p at p + (p >> 4): lanes writing E consecutive positions do not share a bank
+    const MergeLane* mtab;   // [level][lane], of the CTA
     float* col;        // [column][NG]: the mix's gas columns
     float2* kg;        // [gas with a table][NG]: k and dk/dT of the layer's gases
 };
 __host__ __device__ constexpr int pass_chunk(int ng) { return (ng * ng + 31) / 32; }
-__host__ __device__ constexpr int pass_rec_offset(int ng) { return 8 * 32 * pass_chunk(ng); }
-__host__ __device__ constexpr int pass_word_offset(int ng) { return pass_rec_offset(ng) + 8 * (32 * pass_chunk(ng) + 2); }
-__host__ __device__ constexpr int pass_kg_offset(int ng) { return pass_word_offset(ng) + 4 * (34 * pass_chunk(ng) + 2); }
+// gd and rec each hold NG rows of NG + 1 words
+__host__ __device__ constexpr int pass_gd_bytes(int ng) {
+    return 8 * 32 * pass_chunk(ng) > 4 * ng * (ng + 1) ? 8 * 32 * pass_chunk(ng) : (4 * ng * (ng + 1) + 15) & ~15;
+}
+__host__ __device__ constexpr int pass_kg_offset(int ng) { return 2 * pass_gd_bytes(ng) + 16; }
 __host__ __device__ constexpr int pass_scratch_bytes(int ng, int ncol, int ngk) {
     return (pass_kg_offset(ng) + 8 * ngk * ng + 4 * ncol * ng + 15) & ~15;
 }
@@ -268,8 +372,8 @@ __device__ __forceinline__ void walk_bins(const PassScratch& ps, int ng, int nlo
 //
 // The words leave out the low bits of the keys, so two elements whose keys
 // differ only there may come out in the wrong order; the exact keys of every
-// neighbouring pair are compared, and if one is wrong (0.4 % of the passes of
-// the synthetic configurations) the network runs once more on words made of
+// neighbouring pair are compared, and if one is wrong (0.3 % of the passes of
+// the synthetic configurations) the rows are merged once more on words made of
 // the first position of each group of equal leading bits and the low bits,
 // which order the elements exactly, equal keys by element.
 template <int E, int NGC>
@@ -278,7 +382,9 @@ __device__ __forceinline__ void sort_pass(const BatchDev& B, const PassScratch& 
                                           float& cAdd, int lane, Diag& dgn, int dbg_rec) {
     const int ng = NGC ? NGC : ng_run, nloop = NGC ? NGC * NGC : ng_run * ng_run;
     const float kMax = 3.402823466e38f;
-    float x[E];
+    constexpr unsigned kTop = (E ? kPad : kEnd) >> kIdBits;   // leading bits stay below
+    constexpr int kBits = E ? 21 : 22;
+    float x[E ? E : 1];
     bool exact = false, disjoint = false;
     // the smallest key's bits, and how many low bits of key - smallest key the words leave out
     auto key_range = [&](unsigned& smin, int& sh) {
@@ -287,8 +393,8 @@ __device__ __forceinline__ void sort_pass(const BatchDev& B, const PassScratch& 
         const float amax = __uint_as_float(__reduce_max_sync(kFull, lane < ng ? abits : 0u));
         smin = __float_as_uint(__fadd_rn(amin, __shfl_sync(kFull, b, 0)));
         const unsigned range = __float_as_uint(__fadd_rn(amax, __shfl_sync(kFull, b, ng - 1))) - smin;
-        sh = max(0, 32 - __clz(range) - 21);
-        if ((range >> sh) > 0x1fdffeu) ++sh;
+        sh = max(0, 32 - __clz(range) - kBits);
+        if ((range >> sh) >= kTop) ++sh;
     };
     // ---- words -------------------------------------------------------------
     // inputs not monotone in g, negative, infinite or NaN, and keys spread over
@@ -310,48 +416,39 @@ __device__ __forceinline__ void sort_pass(const BatchDev& B, const PassScratch& 
     const int ch = (nloop + 31) >> 5;            // sorted positions a lane runs over below, pads at the end
     const int c0 = lane * ch;
     if (lane >= ng) a = __int_as_float(0x7fffffff);   // a pad's key: NaN, neither below nor equal to any
+    unsigned* gw = (unsigned*)ps.gd;
+    unsigned* rw = (unsigned*)ps.rec;
+    int levels = 0;
+    while ((ng << levels) < nloop) ++levels;
+    unsigned* rows = (levels & 1) ? gw : rw;     // where the merge reads the rows
     if (disjoint) {
 #pragma unroll 1
         for (int p = lane; p < 32 * ch; p += 32) {
             const int i = p / ng;
-            ps.word[p + (p >> 4)] = p < nloop ? (unsigned)(i << 5 | (p - i * ng)) : kIdMask;
+            ps.rec[p].y = p < nloop ? (unsigned)(i << 5 | (p - i * ng)) : kIdMask;
         }
     } else if (net) {
         const unsigned mul = 1u << (kIdBits - sh), sub = smin * mul;
-        if (NGC == 20 && E == 16) {
-            // lane (r, c) of 5 x 5 takes the block of rows 4r.., columns 4c..: rows of four words in order
-            const int r = lane / 5, c = lane - 5 * r;
-            const bool live = lane < 25;
-            const unsigned mask = live ? ~kIdMask : 0u;
-            const unsigned base = live ? (unsigned)((r << 7) | (c << 2)) : (kPadWord | (20u << 5) | 20u);
-            float ar[4], bc[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                ar[q] = __shfl_sync(kFull, a, 4 * r + q);
-                bc[q] = __shfl_sync(kFull, b, 4 * c + q);
-            }
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-#pragma unroll
-                for (int s = 0; s < 4; ++s) {
-                    const unsigned kb = __float_as_uint(__fadd_rn(ar[q], bc[s]));
-                    x[4 * q + s] = __uint_as_float((((kb * mul - sub) & mask) | base) + (unsigned)(32 * q + s));
-                }
-        } else {
+        if (E) {
             int i = lane / ng, j = lane - i * ng;
             const int di = 32 / ng, dj = 32 - di * ng;
 #pragma unroll
             for (int t = 0; t < E; ++t) {
-                const float key = __fadd_rn(__shfl_sync(kFull, a, i), __shfl_sync(kFull, b, j));
-                const unsigned kb = __float_as_uint(key);
-                x[t] = __uint_as_float(t * 32 + lane < nloop ? (((kb * mul - sub) & ~kIdMask) | (unsigned)(i << 5 | j))
-                                                              : (kPadWord | kIdMask));
+                const unsigned kb = __float_as_uint(__fadd_rn(__shfl_sync(kFull, a, i), __shfl_sync(kFull, b, j)));
+                x[t] = __uint_as_float(t * 32 + lane < nloop ? ((kb * mul - sub) & ~kIdMask) | (unsigned)(i << 5 | j) : kPad);
                 j += dj;
                 i += di;
                 if (j >= ng) {
                     j -= ng;
                     ++i;
                 }
+            }
+        } else {
+#pragma unroll 4
+            for (int i = 0; i < ng; ++i) {
+                const unsigned kb = __float_as_uint(__fadd_rn(__shfl_sync(kFull, a, i), b));
+                if (lane <= ng)
+                    rows[i * (ng + 1) + lane] = lane < ng ? ((kb * mul - sub) & ~kIdMask) | (unsigned)(i << 5 | lane) : kEnd;
             }
         }
     }
@@ -372,7 +469,7 @@ __device__ __forceinline__ void sort_pass(const BatchDev& B, const PassScratch& 
 #pragma unroll 1
         for (int p = lane; p < 32 * ch; p += 32) {
             const int e = p < nloop ? (int)(unsigned)W[p] : 0, i = e / ng;
-            ps.word[p + (p >> 4)] = p < nloop ? (unsigned)(i << 5 | (e - i * ng)) : kIdMask;
+            ps.rec[p].y = p < nloop ? (unsigned)(i << 5 | (e - i * ng)) : kIdMask;
         }
         __syncwarp();
         exact = true;
@@ -381,12 +478,12 @@ __device__ __forceinline__ void sort_pass(const BatchDev& B, const PassScratch& 
     if (!net) heapsort_pass();
 
     // ---- sort, cumulative weights, bin boundaries, tie checks ----------------
-    // The sorted words go to shared memory, and each lane runs over a chunk of
-    // consecutive positions: the FP64 prefix of the weights (every partial sum
-    // is exact, so any order gives the reference's values) and the exact keys
-    // of neighbours; a warp scan of the lanes' totals; then lane b finds
-    // boundary b (the first position whose cumulative weight reaches
-    // g_ord(b+1), rankg.f:119-129) and its split fraction.
+    // Each lane runs over a chunk of consecutive sorted positions: the FP64
+    // prefix of the weights (every partial sum is exact, so any order gives the
+    // reference's values) and the exact keys of neighbours; a warp scan of the
+    // lanes' totals; then lane b finds boundary b (the first position whose
+    // cumulative weight reaches g_ord(b+1), rankg.f:119-129) and its split
+    // fraction.
     bool again = false, counted = false;
     int sp, c_last;
     double frac, gprev, tot;
@@ -394,25 +491,35 @@ __device__ __forceinline__ void sort_pass(const BatchDev& B, const PassScratch& 
     unsigned word;
     bool irregular, gerr;
     for (;;) {
-        if (!exact && !disjoint) {
-            warp_sort<E, (NGC == 20 && E == 16) ? 4 : 1>(x, lane);
-#pragma unroll
-            for (int t = 0; t < E; ++t)
-                if (lane * E + t < 32 * ch) ps.word[lane * E + ((lane * E) >> 4) + t] = __float_as_uint(x[t]);
-        }
         __syncwarp();
+        if (!exact && !disjoint) {
+            if (E) {
+                // through gd, position p at p + (p >> 4): lanes writing E consecutive positions do not share a bank
+                warp_sort<E ? E : 1>(x, lane);
+#pragma unroll
+                for (int t = 0; t < E; ++t)
+                    if (lane * E + t < nloop) gw[lane * E + ((lane * E) >> 4) + t] = __float_as_uint(x[t]);
+                __syncwarp();
+                for (int p = lane; p < nloop; p += 32) ps.rec[p].y = gw[p + (p >> 4)];
+            } else {
+                merge_rows<NGC>((unsigned)__cvta_generic_to_shared(gw), (unsigned)__cvta_generic_to_shared(rw), ps.mtab, ng,
+                                levels, lane);
+            }
+            for (int p = nloop + lane; p < 32 * ch; p += 32) ps.rec[p].y = kIdMask;
+            __syncwarp();
+        }
         double run = 0.0;
         bool wrong = false, tie = false;
-        const unsigned qprev = lane > 0 ? ps.word[c0 - 1 + ((c0 - 1) >> 4)] : kIdMask;   // lane 0: a pad
+        const unsigned qprev = lane > 0 ? ps.rec[c0 - 1].y : kIdMask;   // lane 0: a pad
         float kprev = __fadd_rn(__shfl_sync(kFull, a, qprev >> 5), __shfl_sync(kFull, b, qprev));
 #pragma unroll 1
         for (int p = c0; p < c0 + ch; ++p) {
-            const unsigned q = ps.word[p + (p >> 4)];
+            const unsigned q = ps.rec[p].y;
             const float key = __fadd_rn(__shfl_sync(kFull, a, q >> 5), __shfl_sync(kFull, b, q));
             const float w = __fmul_rn(__shfl_sync(kFull, dg, q >> 5), __shfl_sync(kFull, dg, q));
             run = __dadd_rn(run, (double)w);
             ps.gd[p] = run;
-            ps.rec[p] = make_uint2(__float_as_uint(__fmul_rn(key, w)), q);
+            ps.rec[p].x = __float_as_uint(__fmul_rn(key, w));
             wrong |= key < kprev;
             tie |= key == kprev;
             kprev = key;
@@ -424,34 +531,39 @@ __device__ __forceinline__ void sort_pass(const BatchDev& B, const PassScratch& 
             unsigned sm;
             int sb;
             key_range(sm, sb);
-            auto starts = [&](int p, unsigned q) {
-                return p == 0 || ((ps.word[p - 1 + ((p - 1) >> 4)] ^ q) >> kIdBits) != 0;
-            };
+            auto starts = [&](int p, unsigned q) { return p == 0 || ((ps.rec[p - 1].y ^ q) >> kIdBits) != 0; };
             int first = 0;
 #pragma unroll 1
             for (int p = c0; p < min(c0 + ch, nloop); ++p)
-                if (starts(p, ps.word[p + (p >> 4)])) first = p;
+                if (starts(p, ps.rec[p].y)) first = p;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) first = max(first, __shfl_up_sync(kFull, first, o));
             first = __shfl_up_sync(kFull, first, 1);   // of the position before the chunk (lane 0 starts a group)
+            // the new words go to gd, in their rows' order for the merge
             __syncwarp();
-            unsigned* nw = (unsigned*)ps.gd;
 #pragma unroll 1
             for (int p = c0; p < c0 + ch; ++p) {
                 const bool live = p < nloop;
-                const unsigned q = ps.word[p + (p >> 4)];
+                const unsigned q = ps.rec[p].y;
                 const float key = __fadd_rn(__shfl_sync(kFull, a, q >> 5), __shfl_sync(kFull, b, q));
                 if (live) {
                     if (starts(p, q)) first = p;
                     const unsigned rest = (__float_as_uint(key) - sm) & ((1u << sb) - 1);
-                    nw[p] = ((((unsigned)first << sb) | rest) << kIdBits) | (q & kIdMask);
+                    const unsigned w = ((((unsigned)first << sb) | rest) << kIdBits) | (q & kIdMask);
+                    gw[E ? p : ((q >> 5) & 31) * (ng + 1) + (q & 31)] = w;
                 }
             }
             __syncwarp();
+            if (E) {
 #pragma unroll
-            for (int t = 0; t < E; ++t)
-                x[t] = __uint_as_float(lane * E + t < nloop ? nw[lane * E + t] : (kPadWord | kIdMask));
-            __syncwarp();
+                for (int t = 0; t < E; ++t) x[t] = __uint_as_float(lane * E + t < nloop ? gw[lane * E + t] : kPad);
+            } else {
+                if (lane < ng) gw[lane * (ng + 1) + ng] = kEnd;
+                if (rows != gw) {
+                    __syncwarp();
+                    for (int p = lane; p < ng * (ng + 1); p += 32) rw[p] = gw[p];
+                }
+            }
             again = true;
             continue;
         }
