@@ -30,6 +30,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "newton.h"
 
 namespace rtb {
@@ -45,15 +47,17 @@ constexpr int kStage = 2 * kTile;         // hi + lo
 constexpr int kStaging = 2 * kStage + 1024;   // two stages, 1024-byte alignment slack
 constexpr int kStageF64 = 32 * kNp * 8 + 32 * 8;   // hessian_f64: 32 wavenumbers of K in FP64
 
+// C's rows lie an odd number of doubles apart, so a column's lie on different banks
+__host__ __device__ constexpr int c_ld(int nx) { return nx | 1; }
 __host__ __device__ constexpr int cmax(int a, int b) { return a > b ? a : b; }
 // C (nx x nx FP64) aliased with the staging buffers of the pass over K
 __host__ __device__ constexpr int region_bytes(int nx) {
-    return (cmax(nx * nx * 8, cmax(kStaging, kStageF64)) + 15) & ~15;
+    return (cmax(nx * c_ld(nx) * 8, cmax(kStaging, kStageF64)) + 15) & ~15;
 }
-// region + d, rhs, dx, res (kNp doubles each) + the pass's per-warp column
-// partials [kNw][kKc] and the chunk's Se^-1 (dy + K d) [kKc] + 2 mbarriers +
+// region + d, rhs, dx, res, 1 / diag(L) (kNp doubles each) + the pass's per-warp column
+// partials [kNw][kKc], the chunk's Se^-1 (dy + K d) [kKc], Se^-1/2 [2][kKc], 2 mbarriers and
 // the tensor-memory address
-constexpr int kTailBytes = 8 * 4 * kNp + 8 * kNw * kKc + 8 * kKc + 16 + 16;
+constexpr int kTailBytes = 8 * 5 * kNp + 8 * kNw * kKc + 8 * kKc + 4 * 2 * kKc + 16 + 16;
 __host__ __device__ constexpr int newton_smem(int nx) { return region_bytes(nx) + kTailBytes; }
 
 constexpr unsigned kWaitLimit = 1u << 22;
@@ -131,15 +135,17 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-// bf16 round-to-nearest-even of a finite float, as its 16 bits
-__device__ __forceinline__ unsigned bf16_bits(float x) {
-    const unsigned u = __float_as_uint(x);
-    return (u + 0x7fffu + ((u >> 16) & 1u)) >> 16;
+// two floats rounded to bf16 (nearest even), the first in the low half
+__device__ __forceinline__ unsigned bf16_pair(float lo, float hi) {
+    unsigned r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
 }
 
 struct PassSm {
     double* colp;     // [kNw][kKc] per-warp column partials
     double* wch;      // [kKc] Se^-1 (dy + K v) of the chunk
+    float* sc;        // [2][kKc] Se^-1/2 of this chunk and the next
     uint32_t stage0;  // shared address of the first staging stage (1024-aligned)
     uint32_t bar0;    // shared address of the two mbarriers
     uint32_t tmem;    // accumulator address in tensor memory
@@ -153,6 +159,11 @@ struct PassSm {
 // and with kTc the chunk's K~ = Se^-1/2 K goes to shared memory as bf16
 // hi/lo for the tensor-core product N += K~ K~^T.  v and out hold kNp
 // entries (zero beyond nx).  Returns false if an mbarrier wait gave up.
+//
+// Two barriers a chunk bound it, so nothing waits for memory between them: K, y
+// and Se^-1 of the next chunk are read while this one is worked on, and Se^-1/2
+// is formed once per wavenumber.  124 x 2000: about 60 us a pass, where loads
+// at the chunk's own time and a root per element took 100 us.
 template <bool kTc>
 __device__ bool k_pass(const NewtonDev& R, const double* v, bool with_dy, double* out, const PassSm& P) {
     const int nx = R.nx, ny = R.ny;
@@ -161,7 +172,7 @@ __device__ bool k_pass(const NewtonDev& R, const double* v, bool with_dy, double
     double vr[4], acc[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
     for (int r = 0; r < 4; ++r) vr[r] = v[rb + 32 * r];
-    float x[4][8];
+    float x[4][8], xn[4][8];
     auto load = [&](int c) {
         const int nu0 = c * kKc + 8 * g8;
 #pragma unroll
@@ -170,57 +181,74 @@ __device__ bool k_pass(const NewtonDev& R, const double* v, bool with_dy, double
             const float* src = R.kt + (int64_t)row * ny + nu0;
             if (row < nx && nu0 + 8 <= ny && (((uintptr_t)src) & 15) == 0) {
                 const float4 a = __ldg((const float4*)src), b = __ldg((const float4*)src + 1);
-                x[r][0] = a.x; x[r][1] = a.y; x[r][2] = a.z; x[r][3] = a.w;
-                x[r][4] = b.x; x[r][5] = b.y; x[r][6] = b.z; x[r][7] = b.w;
+                xn[r][0] = a.x; xn[r][1] = a.y; xn[r][2] = a.z; xn[r][3] = a.w;
+                xn[r][4] = b.x; xn[r][5] = b.y; xn[r][6] = b.z; xn[r][7] = b.w;
             } else {
 #pragma unroll
-                for (int e = 0; e < 8; ++e) x[r][e] = (row < nx && nu0 + e < ny) ? __ldg(src + e) : 0.0f;
+                for (int e = 0; e < 8; ++e) xn[r][e] = (row < nx && nu0 + e < ny) ? __ldg(src + e) : 0.0f;
             }
         }
+    };
+    // wavenumber tid of a chunk: Se^-1 and the REAL difference y - yn (calcnextxn.f:92)
+    double se = 0.0;
+    float dy = 0.0f;
+    auto load_y = [&](int c) {
+        const int nu = c * kKc + tid;
+        const bool in = tid < kKc && nu < ny;
+        se = in ? R.sei[nu] : 0.0;
+        dy = in && with_dy ? R.y[nu] - R.yn[nu] : 0.0f;
     };
     const int nchunk = (ny + kKc - 1) / kKc;
     bool ok = true;
     uint32_t phase[2] = {0u, 0u};
     load(0);
+    load_y(0);
     for (int c = 0; c < nchunk; ++c) {
-        const int nu0 = c * kKc + 8 * g8;
-        // column partials over this thread's 4 rows, then over the warp's 4 row groups
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) x[r][e] = xn[r][e];
+        if (c + 1 < nchunk) load(c + 1);
+        // column partials over this thread's 4 rows, then over the warp's 4 row
+        // groups: each exchange keeps half of the columns, so lane l ends with two
         double cp[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             double s = 0.0;
 #pragma unroll
             for (int r = 0; r < 4; ++r) s = fma((double)x[r][e], vr[r], s);
-            s += __shfl_xor_sync(0xffffffffu, s, 8);
-            s += __shfl_xor_sync(0xffffffffu, s, 16);
             cp[e] = s;
         }
-        if (lane < 8) {
+        {
+            const bool b3 = lane & 8, b4 = lane & 16;
+            double k4[4], k2[2];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) P.colp[warp * kKc + 8 * g8 + e] = cp[e];
+            for (int e = 0; e < 4; ++e)
+                k4[e] = (b3 ? cp[e + 4] : cp[e]) + __shfl_xor_sync(0xffffffffu, b3 ? cp[e] : cp[e + 4], 8);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                k2[e] = (b4 ? k4[e + 2] : k4[e]) + __shfl_xor_sync(0xffffffffu, b4 ? k4[e] : k4[e + 2], 16);
+                P.colp[warp * kKc + 8 * g8 + (b3 ? 4 : 0) + (b4 ? 2 : 0) + e] = k2[e];
+            }
         }
         const int s = c & 1;
+        if (kTc && tid < kKc) P.sc[s * kKc + tid] = (float)sqrt(se);
         if (kTc && c >= 2) {   // stage s is free once the MMAs of chunk c - 2 are complete
             if (tid == 0 && !mbar_wait(P.bar0 + 8 * s, phase[s])) ok = false;
             phase[s] ^= 1u;
         }
         __syncthreads();
         if (tid < kKc) {
-            const int nu = c * kKc + tid;
-            double w = 0.0;
-            if (nu < ny) {
-                double cs = 0.0;
+            double cs = 0.0;
 #pragma unroll
-                for (int w8 = 0; w8 < kNw; ++w8) cs += P.colp[w8 * kKc + tid];
-                const double dy = with_dy ? (double)(R.y[nu] - R.yn[nu]) : 0.0;   // REAL difference (calcnextxn.f:92)
-                w = (dy + cs) * R.sei[nu];
-            }
-            P.wch[tid] = w;
+            for (int w8 = 0; w8 < kNw; ++w8) cs += P.colp[w8 * kKc + tid];
+            P.wch[tid] = ((double)dy + cs) * se;
         }
+        if (c + 1 < nchunk) load_y(c + 1);
         if (kTc) {
             float sc[8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) sc[e] = nu0 + e < ny ? (float)sqrt(R.sei[nu0 + e]) : 0.0f;
+            for (int e = 0; e < 8; ++e) sc[e] = P.sc[s * kKc + 8 * g8 + e];
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
                 const int row = rb + 32 * r;
@@ -228,10 +256,9 @@ __device__ bool k_pass(const NewtonDev& R, const double* v, bool with_dy, double
 #pragma unroll
                 for (int e = 0; e < 8; e += 2) {
                     const float a = x[r][e] * sc[e], b = x[r][e + 1] * sc[e + 1];
-                    const unsigned ha = bf16_bits(a), hb = bf16_bits(b);
-                    const float ra = a - __uint_as_float(ha << 16), rb2 = b - __uint_as_float(hb << 16);
-                    hi[e / 2] = ha | (hb << 16);
-                    lo[e / 2] = bf16_bits(ra) | (bf16_bits(rb2) << 16);
+                    hi[e / 2] = bf16_pair(a, b);
+                    lo[e / 2] = bf16_pair(a - __uint_as_float(hi[e / 2] << 16),
+                                          b - __uint_as_float(hi[e / 2] & 0xffff0000u));
                 }
                 // row `row`, 16-byte chunk g8, XOR-swizzled by row & 7
                 const uint32_t off = (uint32_t)(row * 128 + ((g8 ^ (row & 7)) << 4));
@@ -266,7 +293,6 @@ __device__ bool k_pass(const NewtonDev& R, const double* v, bool with_dy, double
             for (int e = 0; e < 8; ++e) a = fma((double)x[r][e], P.wch[8 * g8 + e], a);
             acc[r] = a;
         }
-        if (c + 1 < nchunk) load(c + 1);
     }
     if (kTc && tid == 0) {
         // the last commit completes after every MMA of the pass; should it not
@@ -303,7 +329,7 @@ __device__ void c_from_tmem(const NewtonDev& R, uint32_t tmem, double* C) {
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
                 const int col = c0 + 16 * q + i;
-                if (col < nx) C[row * nx + col] = (double)v[i] + R.sai[row * nx + col];
+                if (col < nx) C[row * c_ld(nx) + col] = (double)v[i] + R.sai[row * nx + col];
             }
         }
     }
@@ -349,57 +375,160 @@ __device__ void hessian_f64(const NewtonDev& R, char* sm, double* C) {
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
             const int row = ti * 8 + r, col = tj * 8 + c;
-            if (row < nx && col < nx) C[row * nx + col] = acc[r][c] + R.sai[row * nx + col];
+            if (row < nx && col < nx) C[row * c_ld(nx) + col] = acc[r][c] + R.sai[row * nx + col];
         }
     __syncthreads();
 }
 
-// In-place Cholesky C = L L^T (lower triangle, row-major, stride n).
-// A pivot <= 0 becomes 1 and the factorisation goes on (dcholdc.f:69-84);
-// a NaN pivot propagates as in the reference (sqrt of NaN).
-__device__ bool cholesky(double* C, int n) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+// In-place Cholesky C = L L^T (lower triangle, row-major, stride ld) of n <= 128
+// rows, in panels of 16 columns, by the whole block.  A pivot <= 0 becomes 1 and
+// the factorisation goes on (dcholdc.f:69-84); a NaN pivot propagates as in the
+// reference (sqrt of NaN).  Every element takes its updates in ascending k, one
+// fused multiply-add each, as the column-by-column form does: the same bits.
+// rdiag receives 1 / L(k, k) for the solves.
+//
+// The chain of n square roots and divisions bounds it (about 250 cycles each):
+// one warp runs a panel's 16 x 16 diagonal block on shuffles without a barrier,
+// then every row below divides on its own thread, then the 16 x 16 thread grid
+// updates the rest from registers.  n = 124: 25 us, where column by column with
+// three barriers each took 240 us.
+constexpr int kPanel = 16;
+__device__ bool cholesky(double* C, int n, int ld, double* rdiag) {
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int tx = tid & 15, ty = tid >> 4;
     bool bad = false;
-    for (int k = 0; k < n; ++k) {
-        if (tid == 0) {
-            const double v = C[k * n + k];
-            if (v <= 0.0) {
-                C[k * n + k] = 1.0;
-                bad = true;
-            } else {
-                C[k * n + k] = sqrt(v);
+    for (int k0 = 0; k0 < n; k0 += kPanel) {
+        const int nk = min(kPanel, n - k0);
+        if (tid < 32) {
+            // the diagonal block, row lane (lanes >= nk follow along on row nk - 1 without storing)
+            const int row = min(lane, nk - 1);
+            double c[kPanel];
+#pragma unroll
+            for (int j = 0; j < kPanel; ++j) c[j] = j < nk && j <= row ? C[(k0 + row) * ld + k0 + j] : 0.0;
+#pragma unroll
+            for (int k = 0; k < kPanel; ++k) {
+                if (k < nk) {
+                    const double v = __shfl_sync(0xffffffffu, c[k], k);
+                    bad = bad || v <= 0.0;
+                    const double p = v <= 0.0 ? 1.0 : sqrt(v);
+                    c[k] = row == k ? p : c[k] / p;
+                    if (lane == 0) rdiag[k0 + k] = 1.0 / p;
+#pragma unroll
+                    for (int j = k + 1; j < kPanel; ++j) {
+                        const double ljk = __shfl_sync(0xffffffffu, c[k], j);
+                        c[j] = fma(-c[k], ljk, c[j]);
+                    }
+                }
+            }
+            if (lane < nk) {
+#pragma unroll
+                for (int j = 0; j < kPanel; ++j)
+                    if (j <= lane) C[(k0 + lane) * ld + k0 + j] = c[j];
             }
         }
         __syncthreads();
-        const double p = C[k * n + k];
-        for (int i = k + 1 + tid; i < n; i += kNt) C[i * n + k] = C[i * n + k] / p;
-        __syncthreads();
-        for (int i = k + 1 + warp; i < n; i += kNw) {
-            const double lik = C[i * n + k];
-            for (int j = k + 1 + lane; j <= i; j += 32) C[i * n + j] -= lik * C[j * n + k];
+        const int k1 = k0 + kPanel;
+        if (k1 >= n) break;
+        // the panel's rows below the block, one per thread
+        if (k1 + tid < n) {
+            double* row = C + (k1 + tid) * ld + k0;
+            double c[kPanel];
+#pragma unroll
+            for (int j = 0; j < kPanel; ++j) c[j] = row[j];
+#pragma unroll
+            for (int k = 0; k < kPanel; ++k) {
+                c[k] = c[k] / C[(k0 + k) * ld + k0 + k];
+#pragma unroll
+                for (int j = k + 1; j < kPanel; ++j) c[j] = fma(-c[k], C[(k0 + j) * ld + k0 + k], c[j]);
+            }
+#pragma unroll
+            for (int j = 0; j < kPanel; ++j) row[j] = c[j];
         }
         __syncthreads();
+        // the rest: thread (ty, tx) owns rows k1 + ty + 16 r, columns k1 + tx + 16 q, r >= q
+        constexpr int kB = (kNp - kPanel) / 16;
+        const int nb = (n - k1 + 15) >> 4;
+        double acc[kB][kB];
+#pragma unroll
+        for (int r = 0; r < kB; ++r)
+#pragma unroll
+            for (int q = 0; q <= r; ++q)
+                if (r < nb) {
+                    const int i = k1 + ty + 16 * r, j = k1 + tx + 16 * q;
+                    acc[r][q] = i < n && j <= i ? C[i * ld + j] : 0.0;
+                }
+#pragma unroll 2
+        for (int k = 0; k < kPanel; ++k) {
+            double li[kB], lj[kB];
+#pragma unroll
+            for (int r = 0; r < kB; ++r)
+                if (r < nb) {
+                    li[r] = C[min(k1 + ty + 16 * r, n - 1) * ld + k0 + k];
+                    lj[r] = C[min(k1 + tx + 16 * r, n - 1) * ld + k0 + k];
+                }
+#pragma unroll
+            for (int r = 0; r < kB; ++r)
+#pragma unroll
+                for (int q = 0; q <= r; ++q)
+                    if (r < nb) acc[r][q] = fma(-li[r], lj[q], acc[r][q]);
+        }
+#pragma unroll
+        for (int r = 0; r < kB; ++r)
+#pragma unroll
+            for (int q = 0; q <= r; ++q)
+                if (r < nb) {
+                    const int i = k1 + ty + 16 * r, j = k1 + tx + 16 * q;
+                    if (i < n && j <= i) C[i * ld + j] = acc[r][q];
+                }
+        __syncthreads();
     }
-    return bad;
+    return bad;   // thread 0's is the block's
 }
 
-// Solve L L^T x = b in place in v (one warp; L from cholesky)
-__device__ void chol_solve_warp(const double* L, int n, double* v) {
+// Solve L L^T x = b, lane l holding b and then x at l + 32 r (zero beyond n): one
+// warp, L from cholesky with rdiag its reciprocal diagonal.  The chain of n steps
+// each way bounds it: a shuffle, a multiplication and a fused multiply-add a
+// step, the columns of L read off the chain.
+__device__ __forceinline__ void chol_solve_warp(const double* L, int n, int ld, const double* rdiag, double (&v)[4]) {
     const int lane = threadIdx.x & 31;
-    for (int j = 0; j < n; ++j) {
-        __syncwarp();
-        const double zj = v[j] / L[j * n + j];
-        __syncwarp();
-        if (lane == 0) v[j] = zj;
-        for (int i = j + 1 + lane; i < n; i += 32) v[i] -= L[i * n + j] * zj;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+#pragma unroll 4
+        for (int j = 32 * r; j < min(n, 32 * r + 32); ++j) {
+            const double z = __shfl_sync(0xffffffffu, v[r], j & 31) * rdiag[j];
+            if (lane == (j & 31)) v[r] = z;
+#pragma unroll
+            for (int q = r; q < 4; ++q) {
+                const int i = lane + 32 * q;
+                if (i > j && i < n) v[q] = fma(-L[i * ld + j], z, v[q]);
+            }
+        }
     }
-    for (int j = n - 1; j >= 0; --j) {
-        __syncwarp();
-        const double zj = v[j] / L[j * n + j];
-        __syncwarp();
-        if (lane == 0) v[j] = zj;
-        for (int i = lane; i < j; i += 32) v[i] -= L[j * n + i] * zj;
+#pragma unroll
+    for (int r = 3; r >= 0; --r) {
+#pragma unroll 4
+        for (int j = min(n, 32 * r + 32) - 1; j >= 32 * r; --j) {
+            const double z = __shfl_sync(0xffffffffu, v[r], j & 31) * rdiag[j];
+            if (lane == (j & 31)) v[r] = z;
+#pragma unroll
+            for (int q = 0; q <= r; ++q) {
+                const int i = lane + 32 * q;
+                if (i < j) v[q] = fma(-L[j * ld + i], z, v[q]);
+            }
+        }
     }
+}
+
+// the same on a vector of n entries in shared memory
+__device__ void chol_solve_shared(const double* L, int n, int ld, const double* rdiag, double* b) {
+    const int lane = threadIdx.x & 31;
+    double v[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) v[r] = lane + 32 * r < n ? b[lane + 32 * r] : 0.0;
+    chol_solve_warp(L, n, ld, rdiag, v);
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+        if (lane + 32 * r < n) b[lane + 32 * r] = v[r];
     __syncwarp();
 }
 
@@ -431,9 +560,11 @@ newton_step_kernel(const NewtonDev* __restrict__ rets, int refine, unsigned* __r
     double* dx = rhs + kNp;
     double* res = dx + kNp;
     PassSm P;
-    P.colp = res + kNp;
+    double* rdiag = res + kNp;
+    P.colp = rdiag + kNp;
     P.wch = P.colp + kNw * kKc;
-    uint64_t* bars = (uint64_t*)(P.wch + kKc);
+    P.sc = (float*)(P.wch + kKc);
+    uint64_t* bars = (uint64_t*)(P.sc + 2 * kKc);
     uint32_t* tslot = (uint32_t*)(bars + 2);
     P.stage0 = (smem_u32(smem) + 1023u) & ~1023u;
     P.bar0 = smem_u32(bars);
@@ -471,12 +602,12 @@ newton_step_kernel(const NewtonDev* __restrict__ rets, int refine, unsigned* __r
         hessian_f64(R, smem, C);
         k_pass<false>(R, d, true, rhs, P);
     }
-    const bool bad = cholesky(C, nx);
+    const bool bad = cholesky(C, nx, c_ld(nx), rdiag);
     if (tid == 0 && status) status[blockIdx.x] = bad ? kNtNonPd : 0u;
     // padded entries stay 0: the passes over K read all kNp of them
     for (int i = tid; i < kNp; i += kNt) dx[i] = i < nx ? rhs[i] : 0.0;
     __syncthreads();
-    if (warp == 0) chol_solve_warp(C, nx, dx);
+    if (warp == 0) chol_solve_shared(C, nx, c_ld(nx), rdiag, dx);
     __syncthreads();
     const int nsteps = refine + (resid ? 1 : 0);
     for (int it = 0; it < nsteps; ++it) {
@@ -496,7 +627,7 @@ newton_step_kernel(const NewtonDev* __restrict__ rets, int refine, unsigned* __r
             }
             break;
         }
-        if (warp == 0) chol_solve_warp(C, nx, res);
+        if (warp == 0) chol_solve_shared(C, nx, c_ld(nx), rdiag, res);
         __syncthreads();
         for (int i = tid; i < nx; i += kNt) dx[i] += res[i];
         __syncthreads();
@@ -540,26 +671,32 @@ phi_kernel(const PhiDev* __restrict__ rets, float* __restrict__ phi, float* __re
 }
 
 // Ainv = A^-1 for SPD A (dinvertm.f jmod=2): Cholesky, then one identity
-// column per warp through the two triangular solves.
+// column per warp through the two triangular solves.  The columns of a matrix
+// are split over gridDim.y blocks, each with the (cheaper) factorisation of its
+// own: one 107 x 107 matrix takes 45 us over 14 blocks, where one block that
+// kept its columns in shared memory took 905 us.
 __global__ void __launch_bounds__(kNt, 1)
 spd_inverse_kernel(const double* __restrict__ A, double* __restrict__ Ainv, int n, int64_t stride,
                    unsigned* __restrict__ status) {
     extern __shared__ __align__(16) char smem[];
+    const int ld = c_ld(n);
     double* L = (double*)smem;
-    double* cols = L + n * n;          // [kNw][kNp]
+    double* rdiag = L + n * ld;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const double* a = A + (int64_t)blockIdx.x * stride;
     double* ai = Ainv + (int64_t)blockIdx.x * stride;
-    for (int e = tid; e < n * n; e += kNt) L[e] = a[e];
+    for (int e = tid; e < n * n; e += kNt) L[(e / n) * ld + e % n] = a[e];
     __syncthreads();
-    const bool bad = cholesky(L, n);
-    if (tid == 0 && status) status[blockIdx.x] = bad ? kNtNonPd : 0u;
-    double* v = cols + warp * kNp;
-    for (int j = warp; j < n; j += kNw) {
-        for (int i = lane; i < n; i += 32) v[i] = i == j ? 1.0 : 0.0;
-        chol_solve_warp(L, n, v);
-        for (int i = lane; i < n; i += 32) ai[i * n + j] = v[i];
-        __syncwarp();
+    const bool bad = cholesky(L, n, ld, rdiag);
+    if (tid == 0 && blockIdx.y == 0 && status) status[blockIdx.x] = bad ? kNtNonPd : 0u;
+    for (int j = blockIdx.y * kNw + warp; j < n; j += kNw * gridDim.y) {
+        double v[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) v[r] = lane + 32 * r == j ? 1.0 : 0.0;
+        chol_solve_warp(L, n, ld, rdiag, v);
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+            if (lane + 32 * r < n) ai[(lane + 32 * r) * n + j] = v[r];
     }
 }
 
@@ -591,10 +728,12 @@ cudaError_t launch_phi(const PhiDev* d_ret, int nret, float* d_phi, float* d_chi
 cudaError_t launch_spd_inverse(const double* d_a, double* d_ainv, int n, int64_t stride, int nret,
                                unsigned* d_status, cudaStream_t st) {
     if (nret <= 0) return cudaSuccess;
-    const int smem = n * n * 8 + kNw * kNp * 8;
+    const int smem = n * c_ld(n) * 8 + kNp * 8;
+    // blocks per matrix: one column per warp while the batch leaves SMs idle
+    const int split = std::max(1, std::min((n + kNw - 1) / kNw, 148 / nret));
     cudaError_t e = cudaFuncSetAttribute(spd_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    spd_inverse_kernel<<<nret, kNt, smem, st>>>(d_a, d_ainv, n, stride, d_status);
+    spd_inverse_kernel<<<dim3(nret, split), kNt, smem, st>>>(d_a, d_ainv, n, stride, d_status);
     return cudaGetLastError();
 }
 
