@@ -21,7 +21,7 @@
 //      b. the right-hand side rhs = K^T Se^-1 (y - yn + K d) on the CUDA
 //         cores from the same registers, FP64 accumulation of the FP32 K.
 //      (Alternative: N in FP64 on the CUDA cores, the all-FP64 solve.)
-//   2. C = N + Sa^-1 in FP64 shared memory; Cholesky in FP64 with the
+//   2. C = N + Sa^-1 in FP64 shared memory; LDL^T in FP64 with the
 //      reference's non-positive-pivot rule (pivot 1, continue).
 //   3. dx = C^-1 rhs, then `refine` steps dx += C^-1 (rhs - C_exact dx) where
 //      C_exact applies K^T Se^-1 K through K in FP64 (never through N), one
@@ -54,7 +54,7 @@ __host__ __device__ constexpr int cmax(int a, int b) { return a > b ? a : b; }
 __host__ __device__ constexpr int region_bytes(int nx) {
     return (cmax(nx * c_ld(nx) * 8, cmax(kStaging, kStageF64)) + 15) & ~15;
 }
-// region + d, rhs, dx, res, 1 / diag(L) (kNp doubles each) + the pass's per-warp column
+// region + d, rhs, dx, res, 1 / D (kNp doubles each) + the pass's per-warp column
 // partials [kNw][kKc], the chunk's Se^-1 (dy + K d) [kKc], Se^-1/2 [2][kKc], 2 mbarriers and
 // the tensor-memory address
 constexpr int kTailBytes = 8 * 5 * kNp + 8 * kNw * kKc + 8 * kKc + 4 * 2 * kKc + 16 + 16;
@@ -160,7 +160,8 @@ struct PassSm {
 // hi/lo for the tensor-core product N += K~ K~^T.  v and out hold kNp
 // entries (zero beyond nx).  Returns false if an mbarrier wait gave up.
 //
-// Two barriers a chunk bound it, so nothing waits for memory between them: K, y
+// The conversions of K to FP64 (16 a cycle and SM, each element twice) and two
+// barriers a chunk bound it; nothing waits for memory between the barriers: K, y
 // and Se^-1 of the next chunk are read while this one is worked on, and Se^-1/2
 // is formed once per wavenumber.  124 x 2000: about 60 us a pass, where loads
 // at the chunk's own time and a root per element took 100 us.
@@ -380,20 +381,19 @@ __device__ void hessian_f64(const NewtonDev& R, char* sm, double* C) {
     __syncthreads();
 }
 
-// In-place Cholesky C = L L^T (lower triangle, row-major, stride ld) of n <= 128
-// rows, in panels of 16 columns, by the whole block.  A pivot <= 0 becomes 1 and
-// the factorisation goes on (dcholdc.f:69-84); a NaN pivot propagates as in the
-// reference (sqrt of NaN).  Every element takes its updates in ascending k, one
-// fused multiply-add each, as the column-by-column form does: the same bits.
-// rdiag receives 1 / L(k, k) for the solves.
+// In-place factorisation C = L D L^T (unit L below the diagonal, row-major,
+// stride ld) of n <= 128 rows by the whole block: Cholesky in panels of 16
+// columns, then every column of the factor over its diagonal; rd receives 1 / D.
+// A pivot <= 0 becomes 1 and the factorisation goes on (dcholdc.f:69-84); a NaN
+// pivot propagates as in the reference (root of NaN).
 //
-// The chain of n square roots and divisions bounds it (about 250 cycles each):
-// one warp runs a panel's 16 x 16 diagonal block on shuffles without a barrier,
-// then every row below divides on its own thread, then the 16 x 16 thread grid
-// updates the rest from registers.  n = 124: 25 us, where column by column with
-// three barriers each took 240 us.
+// The chain of n reciprocal roots bounds it: one warp runs a panel's 16 x 16
+// diagonal block on shuffles without a barrier, then every row below goes on its
+// own thread, then the 16 x 16 thread grid updates the rest from registers.  One
+// reciprocal root per column instead of a root and divisions: n = 124 in 63 us
+// with those, column by column with three barriers each 240 us.
 constexpr int kPanel = 16;
-__device__ bool cholesky(double* C, int n, int ld, double* rdiag) {
+__device__ bool factor_ldlt(double* C, int n, int ld, double* rd) {
     const int tid = threadIdx.x, lane = tid & 31;
     const int tx = tid & 15, ty = tid >> 4;
     bool bad = false;
@@ -410,9 +410,9 @@ __device__ bool cholesky(double* C, int n, int ld, double* rdiag) {
                 if (k < nk) {
                     const double v = __shfl_sync(0xffffffffu, c[k], k);
                     bad = bad || v <= 0.0;
-                    const double p = v <= 0.0 ? 1.0 : sqrt(v);
-                    c[k] = row == k ? p : c[k] / p;
-                    if (lane == 0) rdiag[k0 + k] = 1.0 / p;
+                    const double ip = v <= 0.0 ? 1.0 : rsqrt(v);
+                    c[k] *= ip;                       // row k: v / sqrt(v), not used again
+                    if (lane == 0) rd[k0 + k] = ip;
 #pragma unroll
                     for (int j = k + 1; j < kPanel; ++j) {
                         const double ljk = __shfl_sync(0xffffffffu, c[k], j);
@@ -437,7 +437,7 @@ __device__ bool cholesky(double* C, int n, int ld, double* rdiag) {
             for (int j = 0; j < kPanel; ++j) c[j] = row[j];
 #pragma unroll
             for (int k = 0; k < kPanel; ++k) {
-                c[k] = c[k] / C[(k0 + k) * ld + k0 + k];
+                c[k] *= rd[k0 + k];
 #pragma unroll
                 for (int j = k + 1; j < kPanel; ++j) c[j] = fma(-c[k], C[(k0 + j) * ld + k0 + k], c[j]);
             }
@@ -482,50 +482,56 @@ __device__ bool cholesky(double* C, int n, int ld, double* rdiag) {
                 }
         __syncthreads();
     }
+    // L L^T -> L D L^T, eight rows of a column at a time
+    for (int i = tid >> 5; i < n; i += kNw)
+        for (int j = lane; j < i; j += 32) C[i * ld + j] *= rd[j];
+    __syncthreads();
+    for (int i = tid; i < n; i += kNt) rd[i] *= rd[i];
+    __syncthreads();
     return bad;   // thread 0's is the block's
 }
 
-// Solve L L^T x = b, lane l holding b and then x at l + 32 r (zero beyond n): one
-// warp, L from cholesky with rdiag its reciprocal diagonal.  The chain of n steps
-// each way bounds it: a shuffle, a multiplication and a fused multiply-add a
-// step, the columns of L read off the chain.
-__device__ __forceinline__ void chol_solve_warp(const double* L, int n, int ld, const double* rdiag, double (&v)[4]) {
+// Solve L D L^T x = b, lane l holding b and then x at l + 32 r (zero beyond n): one
+// warp.  The chain of n steps each way bounds it: a shuffle and a fused
+// multiply-add a step, the columns of L read off the chain.
+__device__ __forceinline__ void ldlt_solve_warp(const double* L, int n, int ld, const double* rd, double (&v)[4]) {
     const int lane = threadIdx.x & 31;
+    // rows beyond n repeat row n - 1: their entries are never a pivot and never stored
+    const double* row[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) row[q] = L + min(lane + 32 * q, n - 1) * ld;
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
 #pragma unroll 4
         for (int j = 32 * r; j < min(n, 32 * r + 32); ++j) {
-            const double z = __shfl_sync(0xffffffffu, v[r], j & 31) * rdiag[j];
-            if (lane == (j & 31)) v[r] = z;
+            const double z = __shfl_sync(0xffffffffu, v[r], j & 31);
+            if (lane > (j & 31)) v[r] = fma(-row[r][j], z, v[r]);
 #pragma unroll
-            for (int q = r; q < 4; ++q) {
-                const int i = lane + 32 * q;
-                if (i > j && i < n) v[q] = fma(-L[i * ld + j], z, v[q]);
-            }
+            for (int q = r + 1; q < 4; ++q) v[q] = fma(-row[q][j], z, v[q]);
         }
     }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) v[r] = lane + 32 * r < n ? v[r] * rd[lane + 32 * r] : 0.0;
 #pragma unroll
     for (int r = 3; r >= 0; --r) {
 #pragma unroll 4
         for (int j = min(n, 32 * r + 32) - 1; j >= 32 * r; --j) {
-            const double z = __shfl_sync(0xffffffffu, v[r], j & 31) * rdiag[j];
-            if (lane == (j & 31)) v[r] = z;
+            const double z = __shfl_sync(0xffffffffu, v[r], j & 31);
+            const double* col = L + j * ld + lane;
+            if (lane < (j & 31)) v[r] = fma(-col[32 * r], z, v[r]);
 #pragma unroll
-            for (int q = 0; q <= r; ++q) {
-                const int i = lane + 32 * q;
-                if (i < j) v[q] = fma(-L[j * ld + i], z, v[q]);
-            }
+            for (int q = 0; q < r; ++q) v[q] = fma(-col[32 * q], z, v[q]);
         }
     }
 }
 
 // the same on a vector of n entries in shared memory
-__device__ void chol_solve_shared(const double* L, int n, int ld, const double* rdiag, double* b) {
+__device__ void ldlt_solve_shared(const double* L, int n, int ld, const double* rd, double* b) {
     const int lane = threadIdx.x & 31;
     double v[4];
 #pragma unroll
     for (int r = 0; r < 4; ++r) v[r] = lane + 32 * r < n ? b[lane + 32 * r] : 0.0;
-    chol_solve_warp(L, n, ld, rdiag, v);
+    ldlt_solve_warp(L, n, ld, rd, v);
 #pragma unroll
     for (int r = 0; r < 4; ++r)
         if (lane + 32 * r < n) b[lane + 32 * r] = v[r];
@@ -560,8 +566,8 @@ newton_step_kernel(const NewtonDev* __restrict__ rets, int refine, unsigned* __r
     double* dx = rhs + kNp;
     double* res = dx + kNp;
     PassSm P;
-    double* rdiag = res + kNp;
-    P.colp = rdiag + kNp;
+    double* rd = res + kNp;
+    P.colp = rd + kNp;
     P.wch = P.colp + kNw * kKc;
     P.sc = (float*)(P.wch + kKc);
     uint64_t* bars = (uint64_t*)(P.sc + 2 * kKc);
@@ -602,12 +608,12 @@ newton_step_kernel(const NewtonDev* __restrict__ rets, int refine, unsigned* __r
         hessian_f64(R, smem, C);
         k_pass<false>(R, d, true, rhs, P);
     }
-    const bool bad = cholesky(C, nx, c_ld(nx), rdiag);
+    const bool bad = factor_ldlt(C, nx, c_ld(nx), rd);
     if (tid == 0 && status) status[blockIdx.x] = bad ? kNtNonPd : 0u;
     // padded entries stay 0: the passes over K read all kNp of them
     for (int i = tid; i < kNp; i += kNt) dx[i] = i < nx ? rhs[i] : 0.0;
     __syncthreads();
-    if (warp == 0) chol_solve_shared(C, nx, c_ld(nx), rdiag, dx);
+    if (warp == 0) ldlt_solve_shared(C, nx, c_ld(nx), rd, dx);
     __syncthreads();
     const int nsteps = refine + (resid ? 1 : 0);
     for (int it = 0; it < nsteps; ++it) {
@@ -627,7 +633,7 @@ newton_step_kernel(const NewtonDev* __restrict__ rets, int refine, unsigned* __r
             }
             break;
         }
-        if (warp == 0) chol_solve_shared(C, nx, c_ld(nx), rdiag, res);
+        if (warp == 0) ldlt_solve_shared(C, nx, c_ld(nx), rd, res);
         __syncthreads();
         for (int i = tid; i < nx; i += kNt) dx[i] += res[i];
         __syncthreads();
@@ -673,7 +679,7 @@ phi_kernel(const PhiDev* __restrict__ rets, float* __restrict__ phi, float* __re
 // Ainv = A^-1 for SPD A (dinvertm.f jmod=2): Cholesky, then one identity
 // column per warp through the two triangular solves.  The columns of a matrix
 // are split over gridDim.y blocks, each with the (cheaper) factorisation of its
-// own: one 107 x 107 matrix takes 45 us over 14 blocks, where one block that
+// own: one 107 x 107 matrix takes 47 us over 14 blocks, where one block that
 // kept its columns in shared memory took 905 us.
 __global__ void __launch_bounds__(kNt, 1)
 spd_inverse_kernel(const double* __restrict__ A, double* __restrict__ Ainv, int n, int64_t stride,
@@ -681,19 +687,19 @@ spd_inverse_kernel(const double* __restrict__ A, double* __restrict__ Ainv, int 
     extern __shared__ __align__(16) char smem[];
     const int ld = c_ld(n);
     double* L = (double*)smem;
-    double* rdiag = L + n * ld;
+    double* rd = L + n * ld;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const double* a = A + (int64_t)blockIdx.x * stride;
     double* ai = Ainv + (int64_t)blockIdx.x * stride;
     for (int e = tid; e < n * n; e += kNt) L[(e / n) * ld + e % n] = a[e];
     __syncthreads();
-    const bool bad = cholesky(L, n, ld, rdiag);
+    const bool bad = factor_ldlt(L, n, ld, rd);
     if (tid == 0 && blockIdx.y == 0 && status) status[blockIdx.x] = bad ? kNtNonPd : 0u;
     for (int j = blockIdx.y * kNw + warp; j < n; j += kNw * gridDim.y) {
         double v[4];
 #pragma unroll
         for (int r = 0; r < 4; ++r) v[r] = lane + 32 * r == j ? 1.0 : 0.0;
-        chol_solve_warp(L, n, ld, rdiag, v);
+        ldlt_solve_warp(L, n, ld, rd, v);
 #pragma unroll
         for (int r = 0; r < 4; ++r)
             if (lane + 32 * r < n) ai[(lane + 32 * r) * n + j] = v[r];
