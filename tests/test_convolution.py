@@ -158,3 +158,30 @@ def test_cirsrtfg_wave_convolves_outputs(ctx, oracle, mode):
     outs = ctx.cirsrtfg_wave_batch([job, jc, job])
     assert np.array_equal(outs[1][0], c) and np.array_equal(outs[1][1], g) and np.array_equal(outs[1][2], gt)
     assert np.array_equal(outs[0][0], c0) and np.array_equal(outs[2][1], g0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("grid", ["even", "uneven", "repeated", "nan", "steps"])
+@pytest.mark.parametrize("nwave", [2, 3, 66, 514, 515, 1700])
+def test_spline_chunks_match_oracle(ctx, oracle, grid, nwave):
+    """The spline's recurrence in chunks, around one row per thread and more:
+    even, very uneven and repeated abscissae, NaN points, and series of many
+    orders of magnitude.  Within 1e-6 of each series' largest value, as the
+    other FWHM > 0 tests."""
+    rng = np.random.default_rng(nwave)
+    d = np.full(nwave - 1, 0.5)
+    if grid == "uneven":
+        d = 10.0 ** rng.uniform(-2.0, 0.3, nwave - 1)
+    v = (600.0 + np.concatenate([[0.0], np.cumsum(d)])).astype(np.float32)
+    if grid == "repeated" and nwave > 4:
+        v[nwave // 2] = v[nwave // 2 - 1]
+    y = (1.0 + rng.uniform(0.0, 1.0, (3, nwave))).astype(np.float32)
+    if grid == "steps":
+        y = (y * 10.0 ** rng.integers(-12, 1, (3, nwave))).astype(np.float32)
+    if grid == "nan" and nwave > 4:
+        y[1, [1, nwave // 3, nwave - 1]] = np.nan
+    vc = np.linspace(float(v[0]) - 0.3, float(v[-1]) + 0.3, 21).astype(np.float32)
+    got = ctx.cirsconv_ex(v, y, 1.5, Channels(vconv=vc))
+    for s in range(3):
+        ref = oracle.cirsconv_ex(v, y[s], 1.5, Channels(vconv=vc))
+        assert np.max(np.abs(got[s] - ref)) <= 1e-6 * np.max(np.abs(ref)), s
