@@ -198,11 +198,11 @@ struct rtb_context {
     // schedule of the resident batch (rtb_fwd_set_schedule / rtb_fwd_autotune)
     int sched = 0;                        // 0 static, 1 dynamic, 2 dynamic cost-ordered
     int occ = 0;                          // blocks per SM (0 = the occupancy maximum)
-    int tile = rtb::kWarps;               // requested warps per CTA (rtb_fwd_set_tile / rtb_fwd_autotune)
+    int tile = 0;                         // requested warps per CTA (rtb_fwd_set_tile / rtb_fwd_autotune), 0: by the batch
     // the caller's own choices (rtb_fwd_set_tile / rtb_fwd_set_schedule), which a batch of an untuned shape uses
-    int tile_user = rtb::kTileDefault, sched_user = 0, occ_user = 0;
-    int tile_eff = rtb::kWarps;           // warps per CTA of the resident batch's launches
-    int bpsm_w[9] = {};                   // blocks per SM of the batch at 2, 4, 8 warps per CTA (0: not resident)
+    int tile_user = 0, sched_user = 0, occ_user = 0;
+    int tile_eff = rtb::kTileDefault;           // warps per CTA of the resident batch's launches
+    int bpsm_w[rtb::kTileWide + 1] = {};  // blocks per SM of the batch at 2, 4, 8, 16 warps per CTA (0: not resident)
     int bpsm_max = 1;                     // blocks per SM of the current tile
     // rtb_fwd_autotune results by batch shape (layer bucket of 20, gas count): tile, schedule, occupancy
     std::map<std::pair<int, int>, std::array<int, 3>> tuned;

@@ -635,10 +635,9 @@ __device__ __forceinline__ void planck_fp32(int ispace, float vwave, float T, fl
 // fold); otherwise NG is read at run time, and -4 or -8 sort the elements of a
 // pass in that many registers per lane, 0 by merging rows
 template <bool t2, bool ext, int WARPS, int NGC>
-__global__ void __launch_bounds__(WARPS * 32, 24 / WARPS)
+__global__ void __launch_bounds__(WARPS * 32, WARPS <= 8 ? 24 / WARPS : 1)
 fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, int npath_max) {
     constexpr int kThreads = WARPS * 32;
-    constexpr int kWarps = WARPS;
     extern __shared__ __align__(16) char smem[];
     __shared__ SpecDev S_sh;
     const Layout Lo = make_layout(B.ng, nsw_max, ncol_max, ngk_max, nlmax_max, npath_max, WARPS);
@@ -699,7 +698,7 @@ fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, in
             const int* src = (const int*)(B.spec + sidx);
             int* dst = (int*)&S_sh;
             for (int i = tid; i < (int)(sizeof(SpecDev) / sizeof(int)); i += kThreads) dst[i] = src[i];
-            if (tid == 0) s_layer = kWarps;
+            if (tid == 0) s_layer = WARPS;
         }
         __syncthreads();
         const SpecDev& S = S_sh;
@@ -724,7 +723,7 @@ fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, in
         if (B.wg_w2) {
             const float* w2s = B.wg_w2 + S.wg_off + (int64_t)iw * S.ngas;
             const int64_t* slices = B.wg_slice + S.wg_off + (int64_t)iw * S.ngas;
-            for (int l = warp; l < S.nlayer; l += kWarps) {
+            for (int l = warp; l < S.nlayer; l += WARPS) {
                 const KgPos L = kg_pos<t2>(B.lay[S.lay_off + l]);
                 float* ncw = slot() + B.nc_off + ((int64_t)l * S.ngas) * kMaxNg * 2;
                 for (int g = 0; g < S.ngas; ++g)
@@ -855,7 +854,36 @@ fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, in
         const float* tau_s = slot();
         const float* dtau_s = slot_dtau();
         const int nsw = S.nsw;
-        for (int p = warp; p < S.npath; p += kWarps) {
+        // the emission of every layer of the emission paths, and for IMOD 3 its
+        // transmission and absorption per g, spread over the block: a path's own
+        // warp then only runs the products along it
+        for (int p = 0; p < S.npath; ++p) {
+            const int im = S.imod[p], nlays = S.nlayin[p];
+            if (!(im == 3 || (ext && im == 18))) continue;
+            char* ps = region + p * Lo.path_bytes;
+            float* drdt = (float*)(ps + po.drdt);
+            float* trd = (float*)(ps + po.trd);
+            float* bb = (float*)(ps + po.bb);
+            float* dbdt = (float*)(ps + po.dbdt);
+            const int* layinc = B.p_layinc + S.path_off + (int64_t)p * S.nlmax;
+            const float* scale = B.p_scale + S.path_off + (int64_t)p * S.nlmax;
+            const float* emt = B.p_emtemp + S.path_off + (int64_t)p * S.nlmax;
+            for (int j = tid; j < nlays; j += kThreads) {
+                float Tn = emt[j];
+                if (ext && S.inlte)
+                    Tn = nlte_temp(S.inlte, Tn, B.lay_press[S.lp_off + layinc[j]], W.vwave, S.nlte_k1, S.nlte_A);
+                planck_fp32(S.ispace, W.vwave, Tn, bb[j], dbdt[j]);
+            }
+            if (im == 3)
+                for (int t = tid; t < nlays * ng; t += kThreads) {
+                    const int j = t / ng, g = t - j * ng;
+                    const float tau = tau_s[layinc[j] * ng + g] * scale[j];
+                    drdt[t] = expf(-tau);
+                    trd[t] = -expm1f(-tau);
+                }
+        }
+        __syncthreads();
+        for (int p = warp; p < S.npath; p += WARPS) {
             char* ps = region + p * Lo.path_bytes;
             float* drdt = (float*)(ps + po.drdt);
             float* trd = (float*)(ps + po.trd);
@@ -866,24 +894,14 @@ fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, in
             const int nlays = S.nlayin[p], im = S.imod[p];
             const int* layinc = B.p_layinc + S.path_off + (int64_t)p * S.nlmax;
             const float* scale = B.p_scale + S.path_off + (int64_t)p * S.nlmax;
-            const float* emt = B.p_emtemp + S.path_off + (int64_t)p * S.nlmax;
-            if (im == 3 || (ext && im == 18)) {
-                for (int j = lane; j < nlays; j += 32) {
-                    float Tn = emt[j];
-                    if (ext && S.inlte)
-                        Tn = nlte_temp(S.inlte, Tn, B.lay_press[S.lp_off + layinc[j]], W.vwave, S.nlte_k1, S.nlte_A);
-                    planck_fp32(S.ispace, W.vwave, Tn, bb[j], dbdt[j]);
-                }
-            }
-            __syncwarp();
             if (lane < ng) {
                 const int g = lane;
                 if (im == 3) {
                     float tr = 1.0f, R = 0.0f;
+#pragma unroll 4
                     for (int j = 0; j < nlays; ++j) {
-                        const float tau = tau_s[layinc[j] * ng + g] * scale[j];
-                        const float td = -expm1f(-tau) * tr;
-                        const float trn = tr * expf(-tau);
+                        const float td = trd[j * ng + g] * tr;
+                        const float trn = tr * drdt[j * ng + g];
                         R = fmaf(bb[j], td, R);
                         drdt[j * ng + g] = trn;
                         trd[j * ng + g] = td;
@@ -898,6 +916,7 @@ fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, in
                         gt = tr * gg;
                         Ssum = rg * tr;
                     }
+#pragma unroll 4
                     for (int j = nlays - 1; j >= 0; --j) {
                         const float trj = drdt[j * ng + g];
                         drdt[j * ng + g] = bb[j] * trj - Ssum;   // dR/dtau_j
@@ -1006,9 +1025,9 @@ int fwd_smem_bytes(int ng, int nsw, int ncol, int ngk, int nlmax, int npath, int
 
 namespace {
 using FwdKern = void (*)(BatchDev, int, int, int, int, int);
-// the instance of a launch: t2 and ext as the batch needs them; a tile other
-// than kWarps, and NG = 20 as a constant, exist for the usual instance only
-// (one temperature grid, no extended options).  Up to 256 elements a pass are
+// the instance of a launch: t2 and ext as the batch needs them; tiles of 2 and 4
+// warps, and NG = 20 as a constant, exist for the usual instance only (one
+// temperature grid, no extended options).  Up to 256 elements a pass are
 // sorted in registers, more are merged in shared memory: one spectrum of
 // 16-point tables (80 layers, 150 wavenumbers, 2 absorbers) takes 0.22 ms by
 // the first and 0.27 ms by the second, one of 20-point tables (120 layers, 2000
@@ -1021,17 +1040,23 @@ FwdKern fwd_by_ng(int ng) {
     if (ng * ng > 128) return fwd_kernel<t2, ext, WARPS, -8>;
     return fwd_kernel<t2, ext, WARPS, -4>;
 }
+template <int WARPS>
+FwdKern fwd_by_options(bool t2, bool ext, int ng) {
+    if (ext) return t2 ? fwd_by_ng<true, true, WARPS>(ng) : fwd_by_ng<false, true, WARPS>(ng);
+    return fwd_by_ng<true, false, WARPS>(ng);
+}
 FwdKern fwd_instance(bool t2, bool ext, int warps, int ng) {
-    if (ext) return t2 ? fwd_by_ng<true, true, kWarps>(ng) : fwd_by_ng<false, true, kWarps>(ng);
-    if (t2) return fwd_by_ng<true, false, kWarps>(ng);
+    if (ext || t2) return warps == kTileWide ? fwd_by_options<kTileWide>(t2, ext, ng) : fwd_by_options<kTileDefault>(t2, ext, ng);
     if (warps == 2) return fwd_by_ng<false, false, 2>(ng);
-    if (warps == 8) return fwd_by_ng<false, false, 8>(ng);
-    return fwd_by_ng<false, false, kWarps>(ng);
+    if (warps == 4) return fwd_by_ng<false, false, 4>(ng);
+    if (warps == kTileWide) return fwd_by_ng<false, false, kTileWide>(ng);
+    return fwd_by_ng<false, false, kTileDefault>(ng);
 }
 }  // namespace
 
 int fwd_tile_warps(bool t2, bool ext, int warps) {
-    return (ext || t2 || (warps != 2 && warps != 8)) ? kWarps : warps;
+    if (warps == kTileWide) return warps;
+    return (ext || t2 || (warps != 2 && warps != 4)) ? kTileDefault : warps;
 }
 
 int fwd_blocks_per_sm(int smem, bool t2, bool ext, int warps, int ng) {

@@ -1017,16 +1017,16 @@ int prepare_ex(rtb_context* c, int nspec, const rtb_atm* atms, const OutPlace* p
     CUDA_TRY(c, cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
     const bool t2 = c->nt < 0, ext = st.any_para || st.any_ext;
     int bpsm_all = 0;
-    for (int w : {2, 4, 8}) {
+    for (int w : {2, 4, 8, kTileWide}) {
         const int sm_w = fwd_smem_bytes(c->ng, st.nsw_max, st.ncol_max, st.ngk_max, st.nlmax_max, st.npath_max, w);
         c->bpsm_w[w] =
             (sm_w <= smem_max && fwd_tile_warps(t2, ext, w) == w) ? fwd_blocks_per_sm(sm_w, t2, ext, w, c->ng) : 0;
         bpsm_all = std::max(bpsm_all, c->bpsm_w[w]);
     }
-    const int smem = fwd_smem_bytes(c->ng, st.nsw_max, st.ncol_max, st.ngk_max, st.nlmax_max, st.npath_max, kWarps);
+    const int smem = fwd_smem_bytes(c->ng, st.nsw_max, st.ncol_max, st.ngk_max, st.nlmax_max, st.npath_max, kTileDefault);
     if (smem > smem_max)
         return fail(c, RTB_ERR_UNSUPPORTED, "spectrum needs %d B of shared memory (device %d)", smem, smem_max);
-    if (c->bpsm_w[kWarps] <= 0) return fail(c, RTB_ERR_CUDA, "forward kernel cannot be resident (smem %d B)", smem);
+    if (c->bpsm_w[kTileDefault] <= 0) return fail(c, RTB_ERR_CUDA, "forward kernel cannot be resident (smem %d B)", smem);
     // first device spectrum of each caller spectrum (path groups follow it)
     std::vector<int> first(nspec + 1, 0);
     for (int sp = 0; sp < nspec; ++sp) first[sp + 1] = first[sp] + st.nsub[sp];
@@ -1159,8 +1159,8 @@ int prepare_ex(rtb_context* c, int nspec, const rtb_atm* atms, const OutPlace* p
     int64_t grid = (int64_t)c->nsm * bpsm_all;
     if (grid > B.nitems) grid = B.nitems;
     c->grid = (int)grid;
-    c->tile_eff = kWarps;
-    c->bpsm_max = c->bpsm_w[kWarps];
+    c->tile_eff = kTileDefault;
+    c->bpsm_max = c->bpsm_w[kTileDefault];
     // one scratch slot per CTA: tau[Lmax][ng] + dtau[Lmax][nsw][ng]
     B.cell_Lmax = st.Lmax;
     B.cell_slot = (int64_t)st.Lmax * c->ng * (1 + st.nsw_max);
@@ -1234,8 +1234,10 @@ void drop_graph(rtb_context* c) {
 int apply_schedule(rtb_context* c) {
     drop_graph(c);
     BatchDev& B = c->B;
-    const int w = fwd_tile_warps(B.t2, B.ext, c->tile);
-    c->tile_eff = c->bpsm_w[w] > 0 ? w : kWarps;
+    // with an SM or more for every item the layers of one run on twice the warps:
+    // one wavenumber of 40 layers and 2 absorbers takes 89 us by 8 warps, @@ by 16
+    const int w = fwd_tile_warps(B.t2, B.ext, c->tile ? c->tile : (B.nitems <= c->nsm ? kTileWide : kTileDefault));
+    c->tile_eff = c->bpsm_w[w] > 0 ? w : kTileDefault;
     c->bpsm_max = c->bpsm_w[c->tile_eff];
     const int b = c->occ > 0 ? std::min(c->occ, c->bpsm_max) : c->bpsm_max;
     int64_t grid = (int64_t)c->nsm * b;
@@ -1736,7 +1738,7 @@ int rtb_fwd_set_tile(rtb_context* c, int warps) {
     if (!c) return RTB_ERR_ARG;
     if (!(warps == 0 || warps == 2 || warps == 4 || warps == 8))
         return fail(c, RTB_ERR_ARG, "tile of %d warps per block (2, 4 or 8)", warps);
-    c->tile = c->tile_user = warps ? warps : kTileDefault;
+    c->tile = c->tile_user = warps;
     if (!c->prepared) return RTB_OK;
     CUDA_TRY(c, cudaSetDevice(c->device));
     return apply_schedule(c);
@@ -1749,7 +1751,7 @@ int rtb_fwd_autotune(rtb_context* c, rtb_fwd_tune* out) {
     const int keep_graph = c->use_graph;
     c->use_graph = 0;
     float best = 3.4e38f;
-    int best_w = kWarps, best_s = 0, best_b = c->bpsm_w[kWarps], n = 0;
+    int best_w = kTileDefault, best_s = 0, best_b = c->bpsm_w[kTileDefault], n = 0;
     for (int w : {4, 8, 2}) {
         if (fwd_tile_warps(c->B.t2, c->B.ext, w) != w || c->bpsm_w[w] <= 0) continue;
         const int bmax = c->bpsm_w[w];
