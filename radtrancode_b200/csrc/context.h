@@ -19,6 +19,9 @@ int fwd_smem_bytes(int ng, int nsw, int ncol, int ngk, int nlmax, int npath, int
 // warps per CTA a launch uses for a requested tile (tiles other than kWarps
 // exist for the usual instance only), and the blocks per SM it can hold
 int fwd_tile_warps(bool t2, bool ext, int warps);
+// the overlap merge's per-level, per-lane table of an NG (MergeLane)
+size_t fwd_merge_table_bytes();
+void fwd_merge_table(int ng, void* table);
 int fwd_blocks_per_sm(int smem, bool t2, bool ext, int warps, int ng);
 cudaError_t launch_fwd(const BatchDev& B, int nsw, int ncol, int ngk, int nlmax, int npath, int grid, int warps,
                        cudaStream_t st);
@@ -152,7 +155,7 @@ struct rtb_context {
     std::vector<float> vcen;                 // irregular grids: the first table's centres VCEN(NPOINT)
     std::vector<int> tab_id, tab_iso;        // the tables' gas and isotope ids (RTB_KTAB_BY_ID), empty: unknown
     std::vector<std::vector<uint8_t>> nonzero;  // [tab][bin]: bit 0 any value > 0 (get_kg.f:228-250), bit 1 kSliceLog
-    rtb::DevBuf d_raw, d_log, d_delg, d_gord;
+    rtb::DevBuf d_raw, d_log, d_delg, d_gord, d_merge;
     // CIA
     int has_cia = 0;
     float dnu = 0.0f;
@@ -196,11 +199,12 @@ struct rtb_context {
     rtb_fwd_stats stats{};
     int launched_grid = 0;                // blocks of the last forward launch
     // schedule of the resident batch (rtb_fwd_set_schedule / rtb_fwd_autotune)
-    int sched = 0;                        // 0 static, 1 dynamic, 2 dynamic cost-ordered
+    int sched = -1;                       // 0 static, 1 dynamic, 2 dynamic cost-ordered, -1 by the batch
+    const int* order_first = nullptr;     // device: the batch's items longest first (several spectra)
     int occ = 0;                          // blocks per SM (0 = the occupancy maximum)
     int tile = 0;                         // requested warps per CTA (rtb_fwd_set_tile / rtb_fwd_autotune), 0: by the batch
     // the caller's own choices (rtb_fwd_set_tile / rtb_fwd_set_schedule), which a batch of an untuned shape uses
-    int tile_user = 0, sched_user = 0, occ_user = 0;
+    int tile_user = 0, sched_user = -1, occ_user = 0;
     int tile_eff = rtb::kTileDefault;           // warps per CTA of the resident batch's launches
     int bpsm_w[rtb::kTileWide + 1] = {};  // blocks per SM of the batch at 2, 4, 8, 16 warps per CTA (0: not resident)
     int bpsm_max = 1;                     // blocks per SM of the current tile

@@ -645,7 +645,10 @@ fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, in
     float* delg = (float*)(smem + Lo.off_delg);
     char* region = smem + Lo.off_region;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int NG = NGC > 0 ? NGC : 0, E = NGC < 0 ? -NGC : 0;
+    constexpr int NG = NGC > 0 ? NGC : 0;
+    // the wide tile, whose calls wait on latency, sorts in registers at any NG: 2700
+    // cycles a sort of 400 on one warp, the merge 8100
+    constexpr int E = NGC < 0 ? -NGC : WARPS > kTileDefault ? 16 : 0;
     const int ng = NG ? NG : B.ng;     // NGC > 0: the instance for NG = NGC (== B.ng)
     // per-CTA scratch slot in global memory (L2-resident): tau[l][g], dtau[l][s][g]
     auto slot = [&]() { return B.cell_scratch + (int64_t)blockIdx.x * B.cell_slot; };
@@ -654,7 +657,8 @@ fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, in
     const float dg = lane < ng ? B.delg[lane] : 0.0f;                // this lane's g-ordinate weight
     const double gb = lane < ng ? B.g_ord[lane + 1] : 0.0;          // and upper bin boundary
     MergeLane* mtab = (MergeLane*)(smem + Lo.off_mtab);
-    for (int i = tid; i < kMergeLevels * 32; i += kThreads) mtab[i] = merge_lane(ng, i / 32, i % 32);
+    if (E == 0)
+        for (int i = tid; i < kMergeLevels * 32; i += kThreads) ((uint4*)mtab)[i] = ((const uint4*)B.merge_table)[i];
     __shared__ unsigned long long s_count[5];
     if (tid < 5) s_count[tid] = 0;
     __syncthreads();
@@ -751,7 +755,8 @@ fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, in
         for (int l = warp; l < S.nlayer; l = next_layer()) {
             // addresses are formed where they are used: what lives across the
             // overlap passes costs registers, and those bound the resident warps
-            auto amo = [&](int g) { return B.amo[S.lg_off + (int64_t)l * S.ngas + g]; };
+            const float amo_lane = lane < S.ngas ? B.amo[S.lg_off + (int64_t)l * S.ngas + lane] : 0.0f;
+            auto amo = [&](int g) { return __shfl_sync(kFull, amo_lane, g); };
             // k and dk/dT of every gas with a table, (gas, g) spread over the lanes
             {
                 const KgPos L = kg_pos<t2>(B.lay[S.lay_off + l]);
@@ -1019,6 +1024,11 @@ fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, in
 }
 
 // host-side helpers exported to host.cu
+size_t fwd_merge_table_bytes() { return sizeof(MergeLane) * kMergeLevels * 32; }
+void fwd_merge_table(int ng, void* table) {
+    for (int i = 0; i < kMergeLevels * 32; ++i) ((MergeLane*)table)[i] = merge_lane(ng, i / 32, i % 32);
+}
+
 int fwd_smem_bytes(int ng, int nsw, int ncol, int ngk, int nlmax, int npath, int warps) {
     return make_layout(ng, nsw, ncol, ngk, nlmax, npath, warps).total;
 }

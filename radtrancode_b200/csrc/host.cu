@@ -994,6 +994,18 @@ size_t bytes_of(const std::vector<T>& v) {
 cudaStream_t stream_of(rtb_context* c) { return c->user_stream ? c->user_stream : c->stream; }
 
 // pack + upload a batch; the device copy stays resident until the next prepare
+// the items of the resident batch, longest-processing-time first: spectra by
+// decreasing item cost, items of a spectrum together
+static void longest_first(const rtb_context* c, std::vector<int>& order) {
+    const int nspec = (int)c->spec_cost.size();
+    std::vector<int> sp(nspec);
+    for (int i = 0; i < nspec; ++i) sp[i] = i;
+    std::stable_sort(sp.begin(), sp.end(), [&](int a, int b) { return c->spec_cost[a] > c->spec_cost[b]; });
+    order.reserve((size_t)c->item_start_host.back());
+    for (int s : sp)
+        for (int64_t it = c->item_start_host[s]; it < c->item_start_host[s + 1]; ++it) order.push_back((int)it);
+}
+
 int prepare_ex(rtb_context* c, int nspec, const rtb_atm* atms, const OutPlace* place) {
     if (!c || nspec <= 0 || !atms) return fail(c, RTB_ERR_ARG, "bad batch arguments");
     if (c->ntab <= 0) return fail(c, RTB_ERR_NOTABLE, "no k-tables loaded");
@@ -1037,6 +1049,19 @@ int prepare_ex(rtb_context* c, int nspec, const rtb_atm* atms, const OutPlace* p
                 st.spec[k].out_off = place->out_off[sp] + (int64_t)p0 * atms[sp].nwave;
                 st.spec[k].jac_off = place->jac_off[sp] + (int64_t)p0 * atms[sp].nv * atms[sp].nwave;
             }
+    // cost model of one item (wavenumber): layers x (1 + sorting overlap passes) x gradient columns
+    c->spec_cost.clear();
+    for (int s = 0; s < nspec; ++s) {
+        int nabs = 0;
+        for (int k = 0; k < atms[s].ngas; ++k)
+            nabs += (atms[s].ktab[k] >= 0 || atms[s].ktab[k] == RTB_KTAB_BY_ID) ? 1 : 0;
+        for (int k = first[s]; k < first[s + 1]; ++k)   // per device spectrum, as item_start_host
+            c->spec_cost.push_back((float)atms[s].nlayer * (1.0f + 4.0f * std::max(nabs - 1, 0)) *
+                                   (2.0f + st.spec[k].nsw));
+    }
+    c->item_start_host = st.item_start;
+    std::vector<int> order;
+    if (nspec > 1) longest_first(c, order);
     struct Seg {
         const void* src;
         size_t n;
@@ -1071,6 +1096,7 @@ int prepare_ex(rtb_context* c, int nspec, const rtb_atm* atms, const OutPlace* p
     const size_t i_lp = add(st.lpress.data(), bytes_of(st.lpress));
     const size_t i_lt = add(st.ltemp.data(), bytes_of(st.ltemp));
     const size_t i_wf = add(st.wfac.data(), bytes_of(st.wfac));
+    const size_t i_ord = add(order.data(), bytes_of(order));
     const size_t in_bytes = off + 256;
     CUDA_TRY(c, c->h_in.ensure(in_bytes));
     CUDA_TRY(c, c->d_in.ensure(in_bytes));
@@ -1113,6 +1139,7 @@ int prepare_ex(rtb_context* c, int nspec, const rtb_atm* atms, const OutPlace* p
     B.ng = c->ng;
     B.delg = (const float*)c->d_delg.p;
     B.g_ord = (const double*)c->d_gord.p;
+    B.merge_table = c->d_merge.p;
     B.kcia = (const float*)c->d_kcia.p;
     B.e3tab = c->has_e3 ? (const double*)c->d_e3.p : nullptr;
     B.para = st.any_para ? 1 : 0;
@@ -1130,6 +1157,7 @@ int prepare_ex(rtb_context* c, int nspec, const rtb_atm* atms, const OutPlace* p
     B.lay_press = st.lpress.empty() ? nullptr : (const float*)dp(i_lp);
     B.lay_temp = st.ltemp.empty() ? nullptr : (const float*)dp(i_lt);
     B.wave_fac = st.wfac.empty() ? nullptr : (const float*)dp(i_wf);
+    c->order_first = order.empty() ? nullptr : (const int*)dp(i_ord);
     if (place) {
         B.calcout = place->calcout;
         B.gradtsurf = place->gradtsurf;
@@ -1184,22 +1212,13 @@ int prepare_ex(rtb_context* c, int nspec, const rtb_atm* atms, const OutPlace* p
     c->spec_nwave.clear();
     c->spec_nlayer.clear();
     c->cells = 0;
-    c->spec_cost.clear();
     for (int s = 0; s < nspec; ++s) {
         c->spec_npath.push_back(atms[s].npath);
         c->spec_nv.push_back(atms[s].nv);
         c->spec_nwave.push_back(atms[s].nwave);
         c->spec_nlayer.push_back(atms[s].nlayer);
         c->cells += (long long)atms[s].nlayer * atms[s].nwave;
-        // cost model of one item (wavenumber): layers x (1 + sorting overlap passes) x gradient columns
-        int nabs = 0;
-        for (int k = 0; k < atms[s].ngas; ++k)
-            nabs += (atms[s].ktab[k] >= 0 || atms[s].ktab[k] == RTB_KTAB_BY_ID) ? 1 : 0;
-        for (int k = first[s]; k < first[s + 1]; ++k)   // per device spectrum, as item_start_host
-            c->spec_cost.push_back((float)atms[s].nlayer * (1.0f + 4.0f * std::max(nabs - 1, 0)) *
-                                   (2.0f + st.spec[k].nsw));
     }
-    c->item_start_host = st.item_start;
     c->order_ready = 0;
     c->n_out = st.n_out;
     c->n_jac = st.n_jac;
@@ -1235,7 +1254,7 @@ int apply_schedule(rtb_context* c) {
     drop_graph(c);
     BatchDev& B = c->B;
     // with an SM or more for every item the layers of one run on twice the warps:
-    // one wavenumber of 40 layers and 2 absorbers takes 89 us by 8 warps, @@ by 16
+    // one wavenumber of 40 layers and 2 absorbers takes 89 us by 8 warps, 61 by 16
     const int w = fwd_tile_warps(B.t2, B.ext, c->tile ? c->tile : (B.nitems <= c->nsm ? kTileWide : kTileDefault));
     c->tile_eff = c->bpsm_w[w] > 0 ? w : kTileDefault;
     c->bpsm_max = c->bpsm_w[c->tile_eff];
@@ -1243,19 +1262,18 @@ int apply_schedule(rtb_context* c) {
     int64_t grid = (int64_t)c->nsm * b;
     if (grid > B.nitems) grid = B.nitems;
     c->grid = (int)std::max<int64_t>(grid, 1);
-    B.work_next = c->sched >= 1 ? (unsigned long long*)((char*)c->d_diag.p + 48) : nullptr;
-    B.item_order = nullptr;
+    // no schedule asked for: from two items a block on they are pulled from the
+    // counter, the longest spectra of several first; below that the counter's
+    // round trip costs more than it evens out.  14 spectra, 7000 items of 444
+    // blocks: 4.20 ms static, 3.82 ms; 5 spectra, 1000 items: 296 and 264 us; one
+    // spectrum of 515 items: 274 and 288 us
+    const bool dynamic = c->sched >= 1 || (c->sched < 0 && B.nitems >= 2 * (int64_t)c->grid);
+    B.work_next = dynamic ? (unsigned long long*)((char*)c->d_diag.p + 48) : nullptr;
+    B.item_order = c->sched < 0 && dynamic ? c->order_first : nullptr;
     if (c->sched == 2) {
         if (!c->order_ready) {
-            // longest-processing-time first: spectra by decreasing item cost, items of a spectrum together
-            const int nspec = (int)c->spec_cost.size();
-            std::vector<int> sp(nspec);
-            for (int i = 0; i < nspec; ++i) sp[i] = i;
-            std::stable_sort(sp.begin(), sp.end(), [&](int a, int b2) { return c->spec_cost[a] > c->spec_cost[b2]; });
             std::vector<int> order;
-            order.reserve((size_t)B.nitems);
-            for (int s : sp)
-                for (int64_t it = c->item_start_host[s]; it < c->item_start_host[s + 1]; ++it) order.push_back((int)it);
+            longest_first(c, order);
             CUDA_TRY(c, c->d_order.ensure(order.size() * sizeof(int)));
             CUDA_TRY(c, cudaMemcpy(c->d_order.p, order.data(), order.size() * sizeof(int), cudaMemcpyHostToDevice));
             c->order_ready = 1;
@@ -1482,6 +1500,7 @@ void rtb_destroy(rtb_context* c) {
     c->d_log.release();
     c->d_delg.release();
     c->d_gord.release();
+    c->d_merge.release();
     c->d_kcia.release();
     c->d_in.release();
     c->d_out.release();
@@ -1605,6 +1624,10 @@ int rtb_set_ktables(rtb_context* c, int ntab, int np, int nt, int ng, const floa
     CUDA_TRY(c, cudaMemcpy(c->d_log.p, lg.data(), (size_t)total * 4, cudaMemcpyHostToDevice));
     CUDA_TRY(c, cudaMemcpy(c->d_delg.p, delg, (size_t)ng * 4, cudaMemcpyHostToDevice));
     CUDA_TRY(c, cudaMemcpy(c->d_gord.p, c->g_ord.data(), (size_t)(ng + 1) * 8, cudaMemcpyHostToDevice));
+    std::vector<char> mt(fwd_merge_table_bytes());
+    fwd_merge_table(ng, mt.data());
+    CUDA_TRY(c, c->d_merge.ensure(mt.size()));
+    CUDA_TRY(c, cudaMemcpy(c->d_merge.p, mt.data(), mt.size(), cudaMemcpyHostToDevice));
     c->ntab = ntab;
     return RTB_OK;
 }

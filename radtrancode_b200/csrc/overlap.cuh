@@ -17,6 +17,8 @@
 #pragma once
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "rtb_common.h"
 
 namespace rtb {
@@ -100,11 +102,13 @@ constexpr int kMergeLevels = 5;   // merge levels of NG <= 32 rows
 struct MergeLane {
     unsigned short a, b, diag, lo, hi, out, len, pad;
 };
-__device__ inline MergeLane merge_lane(int ng, int level, int l) {
+inline MergeLane merge_lane(int ng, int level, int l) {   // on the host, once per set of tables
     const int n = ng * ng, run = ng << level;
     MergeLane M = {0, 0, 0, 0, 0, 0, 0, 0};
     if (run >= n) return M;
     const int two = run << 1, npairs = (n + two - 1) / two;
+    using std::max;
+    using std::min;
     auto start = [&](int q) {                  // first output position of lane q
         if (q >= 32) return n;
         int p = 0;

@@ -132,6 +132,7 @@ struct BatchDev {
     int t2;                      // NT < 0: one temperature grid per pressure (TEMP2)
     const float* delg;           // [ng]
     const double* g_ord;         // [ng+1], g_ord[ng] forced >= 1 (rankg.f:65-67)
+    const void* merge_table;     // MergeLane [level][lane] of the run's NG
     const float* kcia;           // (9,25,1501) Fortran order
     // E3 table of e3interp (IMOD 18): tabtran | tabe3 | egrad, 1001 each
     const double* e3tab;

@@ -1,4 +1,5 @@
-"""The register sort of an overlap pass (csrc/overlap.cuh) on keys that its
+"""The sorts of an overlap pass (csrc/overlap.cuh: in registers, or merging rows,
+by tile and number of g-ordinates) on keys that their
 words, which leave out the keys' low bits, cannot order by themselves, and on
 keys already in order.  Integer results, so no tolerance: the sorted order of
 every pass that is not the reference heapsort's is the stable order of the
@@ -30,19 +31,22 @@ def _tables(kind, ng):
 
 @pytest.mark.parametrize("kind", ["flat", "wide", "apart"])
 @pytest.mark.parametrize("ng", [3, 11, 12, 16, 17, 20, 22])
-def test_order_of_close_keys(ctx, oracle, kind, ng):
+@pytest.mark.parametrize("tile", [0, 8])     # 0: the wide tile, these calls having few wavenumbers
+def test_order_of_close_keys(ctx, oracle, tile, kind, ng):
     kt, cia = _tables(kind, ng), synth.make_cia(ng)
     job = synth.make_job(kt, [synth.CH4, synth.C2H6], nlayer=13, seed=ng, nwave=4)
     job.amount[:, 3] = job.amount[:, 2]            # both gases' columns alike
     ctx.set_ktables(kt)
     ctx.set_cia(cia)
     ctx.set_debug(True)
+    ctx.set_tile(tile)
     try:
         c, g, _ = ctx.cirsrtfg_wave(job)
         perm, split = ctx.debug_bins(job)
         st = ctx.stats()
     finally:
         ctx.set_debug(False)
+        ctx.set_tile(0)
     _, (hperm, hsplit, _) = oracle.cirsrtfg_wave(kt, cia, job, oracle.ORC_MIXED, debug=True)
     assert st["sort_passes"] == int((hperm[..., 0] >= 0).sum()) > 0
     assert np.array_equal(split, hsplit)
