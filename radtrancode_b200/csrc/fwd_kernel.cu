@@ -622,6 +622,11 @@ __device__ __forceinline__ void planck_fp32(int ispace, float vwave, float T, fl
 
 }  // namespace
 
+// all threads of the cluster, with the global memory they wrote before visible to all after
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
 // ---------------------------------------------------------------------------
 // t2: the run's k-tables carry one temperature grid per pressure (NT < 0);
 // ext: some spectrum takes the para-H2 CIA (flagh2p = 1), an IMOD 18 path or
@@ -651,7 +656,9 @@ fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, in
     constexpr int E = NGC < 0 ? -NGC : WARPS > kTileDefault ? 16 : 0;
     const int ng = NG ? NG : B.ng;     // NGC > 0: the instance for NG = NGC (== B.ng)
     // per-CTA scratch slot in global memory (L2-resident): tau[l][g], dtau[l][s][g]
-    auto slot = [&]() { return B.cell_scratch + (int64_t)blockIdx.x * B.cell_slot; };
+    // and per cluster, where several blocks share an item
+    const int csize = WARPS > kTileDefault ? B.cluster : 1, crank = csize > 1 ? (int)(blockIdx.x % csize) : 0;
+    auto slot = [&]() { return B.cell_scratch + (int64_t)(blockIdx.x / csize) * B.cell_slot; };
     auto slot_dtau = [&]() { return slot() + (int64_t)B.cell_Lmax * ng; };
     for (int i = tid; i < ng; i += kThreads) delg[i] = B.delg[i];
     const float dg = lane < ng ? B.delg[lane] : 0.0f;                // this lane's g-ordinate weight
@@ -676,7 +683,7 @@ fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, in
     __shared__ int64_t s_slice[kMaxGasDev];
     __shared__ unsigned char s_gas[kMaxGasDev];
     __shared__ unsigned s_gmask;
-    int k_static = blockIdx.x;      // items are numbered in 32 bits (item_order)
+    int k_static = blockIdx.x / csize;      // items are numbered in 32 bits (item_order)
     for (;;) {
         // next work item: grid-stride, or pulled from the launch's counter
         // (dynamic schedule); item_order maps the issue order to items
@@ -687,7 +694,7 @@ fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, in
             k = s_next;
         } else {
             k = k_static;
-            k_static += gridDim.x;
+            k_static += gridDim.x / csize;
         }
         if (k >= B.nitems) break;
         const int item = B.item_order ? B.item_order[k] : k;
@@ -727,7 +734,7 @@ fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, in
         if (B.wg_w2) {
             const float* w2s = B.wg_w2 + S.wg_off + (int64_t)iw * S.ngas;
             const int64_t* slices = B.wg_slice + S.wg_off + (int64_t)iw * S.ngas;
-            for (int l = warp; l < S.nlayer; l += WARPS) {
+            for (int l = warp * csize + crank; l < S.nlayer; l += WARPS * csize) {
                 const KgPos L = kg_pos<t2>(B.lay[S.lay_off + l]);
                 float* ncw = slot() + B.nc_off + ((int64_t)l * S.ngas) * kMaxNg * 2;
                 for (int g = 0; g < S.ngas; ++g)
@@ -747,12 +754,14 @@ fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, in
         // ---------------- stage A: layers --------------------------------
         Diag dgn{0, 0, 0};
         // the layers' overlap passes differ in length: a warp takes the next layer when it is done with one
-        auto next_layer = [&]() {
-            int l = 0;
+        // (in a cluster, whose warps have a layer or two each, the next in turn)
+        auto next_layer = [&](int l) {
+            if (csize > 1) return l + WARPS * csize;
+            l = 0;
             if (lane == 0) l = atomicAdd(&s_layer, 1);
             return __shfl_sync(kFull, l, 0);
         };
-        for (int l = warp; l < S.nlayer; l = next_layer()) {
+        for (int l = warp * csize + crank; l < S.nlayer; l = next_layer(l)) {
             // addresses are formed where they are used: what lives across the
             // overlap passes costs registers, and those bound the resident warps
             const float amo_lane = lane < S.ngas ? B.amo[S.lg_off + (int64_t)l * S.ngas + lane] : 0.0f;
@@ -851,6 +860,14 @@ fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, in
             atomicAdd(s_count + 2, (unsigned long long)(dgn.block_exact >> 16));
             atomicAdd(s_count + 3, (unsigned long long)dgn.irregular);
             atomicAdd(s_count + 4, (unsigned long long)(dgn.block_exact & 0xffffu));
+        }
+        if (csize > 1) {
+            // every block's layers are in the slot before the first block runs the paths
+            cluster_sync();
+            if (crank > 0) {
+                cluster_sync();
+                continue;
+            }
         }
         __syncthreads();
 
@@ -1019,6 +1036,7 @@ fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, in
             }
         }
         __syncthreads();
+        if (csize > 1) cluster_sync();      // the slot is free for the next item
     }
     if (tid < 5 && s_count[tid]) atomicAdd(B.counters + tid, s_count[tid]);
 }
@@ -1086,8 +1104,22 @@ cudaError_t launch_fwd(const BatchDev& B, int nsw, int ncol, int ngk, int nlmax,
     const FwdKern kern = fwd_instance(B.t2, B.ext, w, B.ng);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    kern<<<grid, w * 32, smem, st>>>(B, nsw, ncol, ngk, nlmax, npath);
-    return cudaGetLastError();
+    if (B.cluster <= 1) {
+        kern<<<grid, w * 32, smem, st>>>(B, nsw, ncol, ngk, nlmax, npath);
+        return cudaGetLastError();
+    }
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = B.cluster;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid * B.cluster);
+    cfg.blockDim = dim3(w * 32);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, B, nsw, ncol, ngk, nlmax, npath);
 }
 
 }  // namespace rtb

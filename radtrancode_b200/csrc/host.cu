@@ -1253,15 +1253,21 @@ void drop_graph(rtb_context* c) {
 int apply_schedule(rtb_context* c) {
     drop_graph(c);
     BatchDev& B = c->B;
-    // with an SM or more for every item the layers of one run on twice the warps:
-    // one wavenumber of 40 layers and 2 absorbers takes 89 us by 8 warps, 61 by 16
-    const int w = fwd_tile_warps(B.t2, B.ext, c->tile ? c->tile : (B.nitems <= c->nsm ? kTileWide : kTileDefault));
+    // With an SM or more for every item the layers of one run on twice the warps
+    // (one wavenumber of 40 layers and 2 absorbers takes 89 us by 8 warps, 61 by
+    // 16), and with two SMs or more on as many blocks of a cluster, up to 8, as
+    // there are SMs for and layers to share (30 us).
+    const bool wide = !c->tile && B.nitems <= c->nsm;
+    const int w = fwd_tile_warps(B.t2, B.ext, c->tile ? c->tile : (wide ? kTileWide : kTileDefault));
     c->tile_eff = c->bpsm_w[w] > 0 ? w : kTileDefault;
     c->bpsm_max = c->bpsm_w[c->tile_eff];
     const int b = c->occ > 0 ? std::min(c->occ, c->bpsm_max) : c->bpsm_max;
     int64_t grid = (int64_t)c->nsm * b;
     if (grid > B.nitems) grid = B.nitems;
     c->grid = (int)std::max<int64_t>(grid, 1);
+    B.cluster = 1;
+    if (wide && c->sched < 1 && c->tile_eff == kTileWide)
+        while (B.cluster < 8 && 2 * B.cluster * B.nitems <= c->nsm && B.cluster < c->Lmax) B.cluster *= 2;
     // no schedule asked for: from two items a block on they are pulled from the
     // counter, the longest spectra of several first; below that the counter's
     // round trip costs more than it evens out.  14 spectra, 7000 items of 444

@@ -168,6 +168,7 @@ struct BatchDev {
     // schedule (autotuned): issue order of the items, and the dynamic
     // work counter (zero at launch; nullptr = static grid-stride)
     const int* item_order;
+    int cluster;                   // blocks that share an item's layers (a thread-block cluster), 1 = none
     unsigned long long* work_next;
     // per-path-position derivatives dR/dq (cirsradg_wave's doutputdq) of every
     // item, [wave][npath][dq_stride] with dq_stride = nlmax x nsw; nullptr = off
