@@ -195,6 +195,8 @@ struct rtb_context {
     rtb::DevBuf d_conv, d_convout;
     rtb::DevBuf d_layer;                  // rtb_layerg inputs, arguments and outputs
     std::vector<char> h_conv;
+    // fwd_blocks_per_sm by (shared bytes, t2, ext, tile, NG): a query of the driver per tile and call otherwise
+    std::map<std::array<int, 5>, int> bpsm_known;
     size_t dbg_perm_n = 0, dbg_split_n = 0;
     rtb_fwd_stats stats{};
     int launched_grid = 0;                // blocks of the last forward launch

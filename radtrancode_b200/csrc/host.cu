@@ -993,7 +993,6 @@ size_t bytes_of(const std::vector<T>& v) {
 
 cudaStream_t stream_of(rtb_context* c) { return c->user_stream ? c->user_stream : c->stream; }
 
-// pack + upload a batch; the device copy stays resident until the next prepare
 // the items of the resident batch, longest-processing-time first: spectra by
 // decreasing item cost, items of a spectrum together
 static void longest_first(const rtb_context* c, std::vector<int>& order) {
@@ -1006,6 +1005,7 @@ static void longest_first(const rtb_context* c, std::vector<int>& order) {
         for (int64_t it = c->item_start_host[s]; it < c->item_start_host[s + 1]; ++it) order.push_back((int)it);
 }
 
+// pack + upload a batch; the device copy stays resident until the next prepare
 int prepare_ex(rtb_context* c, int nspec, const rtb_atm* atms, const OutPlace* place) {
     if (!c || nspec <= 0 || !atms) return fail(c, RTB_ERR_ARG, "bad batch arguments");
     if (c->ntab <= 0) return fail(c, RTB_ERR_NOTABLE, "no k-tables loaded");
@@ -1031,8 +1031,18 @@ int prepare_ex(rtb_context* c, int nspec, const rtb_atm* atms, const OutPlace* p
     int bpsm_all = 0;
     for (int w : {2, 4, 8, kTileWide}) {
         const int sm_w = fwd_smem_bytes(c->ng, st.nsw_max, st.ncol_max, st.ngk_max, st.nlmax_max, st.npath_max, w);
-        c->bpsm_w[w] =
-            (sm_w <= smem_max && fwd_tile_warps(t2, ext, w) == w) ? fwd_blocks_per_sm(sm_w, t2, ext, w, c->ng) : 0;
+        if (sm_w > smem_max || fwd_tile_warps(t2, ext, w) != w) {
+            c->bpsm_w[w] = 0;
+        } else {
+            const std::array<int, 5> key = {sm_w, t2, ext, w, c->ng};
+            const auto known = c->bpsm_known.find(key);
+            if (known != c->bpsm_known.end()) {
+                c->bpsm_w[w] = known->second;
+            } else {
+                c->bpsm_w[w] = fwd_blocks_per_sm(sm_w, t2, ext, w, c->ng);
+                if (c->bpsm_known.size() < 256) c->bpsm_known[key] = c->bpsm_w[w];
+            }
+        }
         bpsm_all = std::max(bpsm_all, c->bpsm_w[w]);
     }
     const int smem = fwd_smem_bytes(c->ng, st.nsw_max, st.ncol_max, st.ngk_max, st.nlmax_max, st.npath_max, kTileDefault);
@@ -1612,16 +1622,15 @@ int rtb_set_ktables(rtb_context* c, int ntab, int np, int nt, int ng, const floa
     for (int t = 0; t < ntab; ++t) {
         c->nonzero[t].assign(nbin[t], 0);
         for (int b = 0; b < nbin[t]; ++b) {
-            const float* s = data + c->tab_off[t] + (int64_t)b * slice;
-            uint8_t any = 0;
-            for (int64_t i = 0; i < slice; ++i)
-                if (s[i] > 0.0f) { any = 1; break; }
-            bool log0 = true;
+            const int64_t at = c->tab_off[t] + (int64_t)b * slice;
+            const float* s = data + at;
+            bool any = false, log0 = true;
+            for (int64_t i = 0; i < slice && !any; ++i) any = s[i] > 0.0f;
+            for (int64_t i = 0; i < slice; ++i) lg[at + i] = (float)std::log((double)s[i]);
             for (int64_t i = 0; i < slice; i += ng) log0 = log0 && !(s[i] <= 0.0f);
-            c->nonzero[t][b] = (uint8_t)(any | (log0 ? 2 : 0));
+            c->nonzero[t][b] = (uint8_t)((any ? 1 : 0) | (log0 ? 2 : 0));
         }
     }
-    for (int64_t i = 0; i < total; ++i) lg[i] = (float)std::log((double)data[i]);
     CUDA_TRY(c, c->d_raw.ensure((size_t)total * 4));
     CUDA_TRY(c, c->d_log.ensure((size_t)total * 4));
     CUDA_TRY(c, c->d_delg.ensure(4 * 64));

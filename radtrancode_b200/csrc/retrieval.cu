@@ -707,8 +707,8 @@ struct Engine {
             std::copy(s->xn.begin(), s->xn.end(), r + kNewtonMaxNx);
             std::copy(s->xn1.begin(), s->xn1.end(), r + 2 * kNewtonMaxNx);
         }
+        // from pageable memory: xs has been read when the call returns
         CUDA_TRY(c, cudaMemcpyAsync(xarea.p, xs.data(), xs.size() * 4, cudaMemcpyHostToDevice, st));
-        CUDA_TRY(c, cudaStreamSynchronize(st));
         return RTB_OK;
     }
 
@@ -807,11 +807,6 @@ struct Engine {
                 CUDA_TRY(c, cudaMemcpy2DAsync(kb + (size_t)p * ny1, (size_t)s->ny * 4, jrow + (size_t)p * s->nx * ny1,
                                               (size_t)ny1 * 4, (size_t)ny1 * 4, s->nx, cudaMemcpyDeviceToDevice, st));
         }
-        CUDA_TRY(c, cudaStreamSynchronize(st));
-        unsigned long long diag[8];
-        CUDA_TRY(c, cudaMemcpy(diag, c->d_diag.p, 64, cudaMemcpyDeviceToHost));
-        if ((unsigned)(diag[0] & 0xffffffffu) & kStGord)
-            return fail(c, RTB_ERR_GORD, "g-ordinate walk ran past NG (rankg.f:118-147)");
         std::vector<PhiDev> desc;
         for (const Slot* s : v) {
             const bool first = s->phase == 0;
@@ -831,8 +826,12 @@ struct Engine {
         float* out = (float*)small.p;
         CUDA_TRY(c, launch_phi((const PhiDev*)phi_desc.p, (int)v.size(), out, out + v.size(), st));
         ph.resize(2 * v.size());
+        unsigned long long diag[8];
         CUDA_TRY(c, cudaMemcpyAsync(ph.data(), out, 8 * v.size(), cudaMemcpyDeviceToHost, st));
+        CUDA_TRY(c, cudaMemcpyAsync(diag, c->d_diag.p, 64, cudaMemcpyDeviceToHost, st));
         CUDA_TRY(c, cudaStreamSynchronize(st));
+        if ((unsigned)(diag[0] & 0xffffffffu) & kStGord)
+            return fail(c, RTB_ERR_GORD, "g-ordinate walk ran past NG (rankg.f:118-147)");
         return RTB_OK;
     }
 
