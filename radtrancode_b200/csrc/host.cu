@@ -1618,25 +1618,31 @@ int rtb_set_ktables(rtb_context* c, int ntab, int np, int nt, int ng, const floa
         c->tab_off[t] = total;
         total += (int64_t)nbin[t] * slice;
     }
-    std::vector<float> lg((size_t)total);
-    for (int t = 0; t < ntab; ++t) {
-        c->nonzero[t].assign(nbin[t], 0);
-        for (int b = 0; b < nbin[t]; ++b) {
-            const int64_t at = c->tab_off[t] + (int64_t)b * slice;
-            const float* s = data + at;
-            bool any = false, log0 = true;
-            for (int64_t i = 0; i < slice && !any; ++i) any = s[i] > 0.0f;
-            for (int64_t i = 0; i < slice; ++i) lg[at + i] = (float)std::log((double)s[i]);
-            for (int64_t i = 0; i < slice; i += ng) log0 = log0 && !(s[i] <= 0.0f);
-            c->nonzero[t][b] = (uint8_t)((any ? 1 : 0) | (log0 ? 2 : 0));
-        }
-    }
     CUDA_TRY(c, c->d_raw.ensure((size_t)total * 4));
     CUDA_TRY(c, c->d_log.ensure((size_t)total * 4));
+    // ln k piece by piece: a vector as large as the tables is 12 ms of page faults for 40 MB
+    std::vector<float> lg((size_t)std::max<int64_t>(slice, 1 << 19));
+    const int nrun = (int)((int64_t)lg.size() / slice);
+    for (int t = 0; t < ntab; ++t) {
+        c->nonzero[t].assign(nbin[t], 0);
+        for (int b0 = 0; b0 < nbin[t]; b0 += nrun) {
+            const int n = std::min(nrun, nbin[t] - b0);
+            for (int b = 0; b < n; ++b) {
+                const float* s = data + c->tab_off[t] + (b0 + b) * slice;
+                float* d = lg.data() + b * slice;
+                bool any = false, log0 = true;
+                for (int64_t i = 0; i < slice && !any; ++i) any = s[i] > 0.0f;
+                for (int64_t i = 0; i < slice; ++i) d[i] = (float)std::log((double)s[i]);
+                for (int64_t i = 0; i < slice; i += ng) log0 = log0 && !(s[i] <= 0.0f);
+                c->nonzero[t][b0 + b] = (uint8_t)((any ? 1 : 0) | (log0 ? 2 : 0));
+            }
+            CUDA_TRY(c, cudaMemcpy((float*)c->d_log.p + c->tab_off[t] + b0 * slice, lg.data(), (size_t)(n * slice) * 4,
+                                   cudaMemcpyHostToDevice));
+        }
+    }
     CUDA_TRY(c, c->d_delg.ensure(4 * 64));
     CUDA_TRY(c, c->d_gord.ensure(8 * 64));
     CUDA_TRY(c, cudaMemcpy(c->d_raw.p, data, (size_t)total * 4, cudaMemcpyHostToDevice));
-    CUDA_TRY(c, cudaMemcpy(c->d_log.p, lg.data(), (size_t)total * 4, cudaMemcpyHostToDevice));
     CUDA_TRY(c, cudaMemcpy(c->d_delg.p, delg, (size_t)ng * 4, cudaMemcpyHostToDevice));
     CUDA_TRY(c, cudaMemcpy(c->d_gord.p, c->g_ord.data(), (size_t)(ng + 1) * 8, cudaMemcpyHostToDevice));
     std::vector<char> mt(fwd_merge_table_bytes());
