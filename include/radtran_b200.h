@@ -401,21 +401,24 @@ int rtb_set_strict_ties(rtb_context* ctx, int on);
  *   schedule 1  dynamic: blocks pull the next item from a counter
  *   schedule 2  dynamic, items issued longest first (spectra ordered by a
  *               cost model: layers x overlap passes x gradient columns)
- * blocks_per_sm 0 = the occupancy maximum.  Results do not depend on the
- * schedule (each item is computed by one block, in the same order). */
+ * blocks_per_sm 0 = the occupancy maximum.  A context in which no schedule was
+ * set chooses: 0 with fewer than two items a block, else 1, or 2 for a batch of
+ * several spectra.  Results do not depend on the schedule. */
 int rtb_fwd_set_schedule(rtb_context* ctx, int schedule, int blocks_per_sm);
 
 /* Tile shape of the resident batch's launches: warps per block, i.e. the
  * layers of one (spectrum, wavenumber) item worked on at once (one warp per
- * layer, one lane per g-ordinate): 2, 4 or 8; 0 = the default 8.  Tiles
- * other than 4 exist for the usual kernel instance (one temperature grid, no
- * para-H2 / IMOD 18 / iform / non-LTE / air-Rayleigh option); other batches
- * run 4.  Results do not depend on the tile. */
+ * layer, one lane per g-ordinate): 2, 4 or 8; 0 (the default) = chosen by the
+ * batch: 8, or 16 where there are no more items than SMs, several blocks sharing
+ * an item where more SMs would be idle.  Tiles 2 and 4 exist for the usual kernel
+ * instance (one temperature grid, no para-H2 / IMOD 18 / iform / non-LTE /
+ * air-Rayleigh option); other batches run 8.  Results do not depend on the tile. */
 int rtb_fwd_set_tile(rtb_context* ctx, int warps);
 
 /* Time the resident batch under every tile (2, 4, 8 warps per block) x
- * schedule x the three highest occupancies of the tile (two launches each,
- * the second timed), keep the fastest and report it.  The result is also
+ * schedule x the three highest occupancies of the tile, and what a batch runs
+ * that nothing was set for (two launches each, the second timed), keep the
+ * fastest and report it.  The result is also
  * kept in the context under the batch's shape (its largest layer count in
  * buckets of 20 layers, and its largest gas count): a later rtb_fwd_prepare
  * of a batch of the same shape starts with it (tune on a representative
@@ -427,7 +430,7 @@ typedef struct rtb_fwd_tune {
     int blocks_per_sm;
     float ms;          /* launch time of the chosen configuration */
     int candidates;    /* configurations timed */
-    int warps;         /* warps per block of the chosen tile */
+    int warps;         /* warps per block of the chosen tile: 2, 4, 8 or 16 */
 } rtb_fwd_tune;
 int rtb_fwd_autotune(rtb_context* ctx, rtb_fwd_tune* out);
 

@@ -639,7 +639,7 @@ __device__ __forceinline__ void cluster_sync() {
 // NG as a compile-time constant (the overlap's sizes, offsets and loop bounds
 // fold); otherwise NG is read at run time, and -4 or -8 sort the elements of a
 // pass in that many registers per lane, 0 by merging rows
-template <bool t2, bool ext, int WARPS, int NGC>
+template <bool t2, bool ext, int WARPS, int NGC, int CL = 1>
 __global__ void __launch_bounds__(WARPS * 32, WARPS <= 8 ? 24 / WARPS : 1)
 fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, int npath_max) {
     constexpr int kThreads = WARPS * 32;
@@ -653,11 +653,11 @@ fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, in
     constexpr int NG = NGC > 0 ? NGC : 0;
     // the wide tile, whose calls wait on latency, sorts in registers at any NG: 2700
     // cycles a sort of 400 on one warp, the merge 8100
-    constexpr int E = NGC < 0 ? -NGC : WARPS > kTileDefault ? 16 : 0;
+    constexpr int E = NGC < 0 ? -NGC : WARPS > kTileDefault || CL > 1 ? 16 : 0;
     const int ng = NG ? NG : B.ng;     // NGC > 0: the instance for NG = NGC (== B.ng)
     // per-CTA scratch slot in global memory (L2-resident): tau[l][g], dtau[l][s][g]
     // and per cluster, where several blocks share an item
-    const int csize = WARPS > kTileDefault ? B.cluster : 1, crank = csize > 1 ? (int)(blockIdx.x % csize) : 0;
+    const int csize = WARPS > kTileDefault ? B.cluster : CL, crank = csize > 1 ? (int)(blockIdx.x % csize) : 0;
     auto slot = [&]() { return B.cell_scratch + (int64_t)(blockIdx.x / csize) * B.cell_slot; };
     auto slot_dtau = [&]() { return slot() + (int64_t)B.cell_Lmax * ng; };
     for (int i = tid; i < ng; i += kThreads) delg[i] = B.delg[i];
@@ -1061,24 +1061,24 @@ using FwdKern = void (*)(BatchDev, int, int, int, int, int);
 // the first and 0.27 ms by the second, one of 20-point tables (120 layers, 2000
 // wavenumbers, 4 absorbers) 3.68 and 3.45 ms.
 constexpr int kNgConst = 20;
-template <bool t2, bool ext, int WARPS>
+template <bool t2, bool ext, int WARPS, int CL = 1>
 FwdKern fwd_by_ng(int ng) {
-    if (!t2 && !ext && ng == kNgConst) return fwd_kernel<t2, ext, WARPS, t2 || ext ? 0 : kNgConst>;
-    if (ng * ng > 256) return fwd_kernel<t2, ext, WARPS, 0>;
-    if (ng * ng > 128) return fwd_kernel<t2, ext, WARPS, -8>;
-    return fwd_kernel<t2, ext, WARPS, -4>;
+    if (!t2 && !ext && ng == kNgConst) return fwd_kernel<t2, ext, WARPS, t2 || ext ? 0 : kNgConst, CL>;
+    if (ng * ng > 256) return fwd_kernel<t2, ext, WARPS, 0, CL>;
+    if (ng * ng > 128) return fwd_kernel<t2, ext, WARPS, -8, CL>;
+    return fwd_kernel<t2, ext, WARPS, -4, CL>;
 }
-template <int WARPS>
+template <int WARPS, int CL = 1>
 FwdKern fwd_by_options(bool t2, bool ext, int ng) {
-    if (ext) return t2 ? fwd_by_ng<true, true, WARPS>(ng) : fwd_by_ng<false, true, WARPS>(ng);
-    return fwd_by_ng<true, false, WARPS>(ng);
+    if (ext) return t2 ? fwd_by_ng<true, true, WARPS, CL>(ng) : fwd_by_ng<false, true, WARPS, CL>(ng);
+    return t2 ? fwd_by_ng<true, false, WARPS, CL>(ng) : fwd_by_ng<false, false, WARPS, CL>(ng);
 }
-FwdKern fwd_instance(bool t2, bool ext, int warps, int ng) {
-    if (ext || t2) return warps == kTileWide ? fwd_by_options<kTileWide>(t2, ext, ng) : fwd_by_options<kTileDefault>(t2, ext, ng);
-    if (warps == 2) return fwd_by_ng<false, false, 2>(ng);
-    if (warps == 4) return fwd_by_ng<false, false, 4>(ng);
-    if (warps == kTileWide) return fwd_by_ng<false, false, kTileWide>(ng);
-    return fwd_by_ng<false, false, kTileDefault>(ng);
+FwdKern fwd_instance(bool t2, bool ext, int warps, int ng, bool pair) {
+    if (warps == kTileWide) return fwd_by_options<kTileWide>(t2, ext, ng);
+    if (pair) return fwd_by_options<kTileDefault, 2>(t2, ext, ng);
+    if (warps == 2 && !t2 && !ext) return fwd_by_ng<false, false, 2>(ng);
+    if (warps == 4 && !t2 && !ext) return fwd_by_ng<false, false, 4>(ng);
+    return fwd_by_options<kTileDefault>(t2, ext, ng);
 }
 }  // namespace
 
@@ -1089,7 +1089,7 @@ int fwd_tile_warps(bool t2, bool ext, int warps) {
 
 int fwd_blocks_per_sm(int smem, bool t2, bool ext, int warps, int ng) {
     const int w = fwd_tile_warps(t2, ext, warps);
-    const FwdKern k = fwd_instance(t2, ext, w, ng);
+    const FwdKern k = fwd_instance(t2, ext, w, ng, false);
     int n = 0;
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, w * 32, smem) != cudaSuccess)
@@ -1101,7 +1101,7 @@ cudaError_t launch_fwd(const BatchDev& B, int nsw, int ncol, int ngk, int nlmax,
                        cudaStream_t st) {
     const int w = fwd_tile_warps(B.t2, B.ext, warps);
     const int smem = fwd_smem_bytes(B.ng, nsw, ncol, ngk, nlmax, npath, w);
-    const FwdKern kern = fwd_instance(B.t2, B.ext, w, B.ng);
+    const FwdKern kern = fwd_instance(B.t2, B.ext, w, B.ng, w == kTileDefault && B.cluster == 2);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     if (B.cluster <= 1) {

@@ -1266,7 +1266,10 @@ int apply_schedule(rtb_context* c) {
     // With an SM or more for every item the layers of one run on twice the warps
     // (one wavenumber of 40 layers and 2 absorbers takes 89 us by 8 warps, 61 by
     // 16), and with two SMs or more on as many blocks of a cluster, up to 8, as
-    // there are SMs for and layers to share (30 us).
+    // there are SMs for and layers to share (30 us).  Beyond that, while two blocks
+    // of 8 warps an item are resident at once, on a pair of them: 80 layers, 16-point
+    // tables, 149 wavenumbers 155 us by one block, 117 by two; 120 layers, 4
+    // absorbers, 222 wavenumbers 592 and 545 us.
     const bool wide = !c->tile && B.nitems <= c->nsm;
     const int w = fwd_tile_warps(B.t2, B.ext, c->tile ? c->tile : (wide ? kTileWide : kTileDefault));
     c->tile_eff = c->bpsm_w[w] > 0 ? w : kTileDefault;
@@ -1278,6 +1281,8 @@ int apply_schedule(rtb_context* c) {
     B.cluster = 1;
     if (wide && c->sched < 1 && c->tile_eff == kTileWide)
         while (B.cluster < 8 && 2 * B.cluster * B.nitems <= c->nsm && B.cluster < c->Lmax) B.cluster *= 2;
+    if (!c->tile && !wide && c->sched < 1 && c->occ <= 0 && 2 * (int64_t)B.nitems <= (int64_t)c->nsm * b)
+        B.cluster = 2;
     // no schedule asked for: from two items a block on they are pulled from the
     // counter, the longest spectra of several first; below that the counter's
     // round trip costs more than it evens out.  14 spectra, 7000 items of 444
@@ -1796,32 +1801,37 @@ int rtb_fwd_autotune(rtb_context* c, rtb_fwd_tune* out) {
     c->use_graph = 0;
     float best = 3.4e38f;
     int best_w = kTileDefault, best_s = 0, best_b = c->bpsm_w[kTileDefault], n = 0;
+    auto time_it = [&](int w, int sch, int b) {
+        c->tile = w;
+        c->sched = sch;
+        c->occ = b;
+        int r = apply_schedule(c);
+        if (r) return r;
+        float ms = 0.0f;
+        for (int rep = 0; rep < 2; ++rep) {   // the second launch is timed
+            r = launch(c);
+            if (r) return r;
+            CUDA_TRY(c, cudaStreamSynchronize(strm));
+            CUDA_TRY(c, cudaEventElapsedTime(&ms, c->ev0, c->ev1));
+        }
+        ++n;
+        if (ms < best) {
+            best = ms;
+            best_w = w;
+            best_s = sch;
+            best_b = b;
+        }
+        return (int)RTB_OK;
+    };
     for (int w : {4, 8, 2}) {
         if (fwd_tile_warps(c->B.t2, c->B.ext, w) != w || c->bpsm_w[w] <= 0) continue;
         const int bmax = c->bpsm_w[w];
         for (int sch = 0; sch <= 2; ++sch)
-            for (int b = bmax; b >= 1 && b >= bmax - 2; --b) {
-                c->tile = w;
-                c->sched = sch;
-                c->occ = b;
-                int r = apply_schedule(c);
-                if (r) return r;
-                float ms = 0.0f;
-                for (int rep = 0; rep < 2; ++rep) {   // the second launch is timed
-                    r = launch(c);
-                    if (r) return r;
-                    CUDA_TRY(c, cudaStreamSynchronize(strm));
-                    CUDA_TRY(c, cudaEventElapsedTime(&ms, c->ev0, c->ev1));
-                }
-                ++n;
-                if (ms < best) {
-                    best = ms;
-                    best_w = w;
-                    best_s = sch;
-                    best_b = b;
-                }
-            }
+            for (int b = bmax; b >= 1 && b >= bmax - 2; --b)
+                if (const int r = time_it(w, sch, b)) return r;
     }
+    // and what a batch that nothing was set for runs
+    if (const int r = time_it(0, -1, 0)) return r;
     c->tile = best_w;
     c->sched = best_s;
     c->occ = best_b;
@@ -1830,11 +1840,11 @@ int rtb_fwd_autotune(rtb_context* c, rtb_fwd_tune* out) {
     const int r = apply_schedule(c);
     if (r) return r;
     if (out) {
-        out->schedule = best_s;
-        out->blocks_per_sm = best_b;
+        out->schedule = best_s >= 0 ? best_s : !c->B.work_next ? 0 : !c->B.item_order ? 1 : 2;
+        out->blocks_per_sm = best_b > 0 ? best_b : c->bpsm_max;
         out->ms = best;
         out->candidates = n;
-        out->warps = best_w;
+        out->warps = c->tile_eff;
     }
     return RTB_OK;
 }

@@ -9,7 +9,7 @@ import os
 import numpy as np
 import pytest
 
-from radtrancode_b200 import synth
+from radtrancode_b200 import cirsradg, synth
 from tests.helpers import JAC_TOL, RAD_TOL, jac_err, rad_err
 
 pytestmark = pytest.mark.gpu
@@ -79,3 +79,53 @@ def test_uneven_batch_against_fp64_oracle(ctx, oracle, uneven):
         assert rad_err(c, c64) <= RAD_TOL
         assert jac_err(g, g64, j.nv) <= JAC_TOL
     print(f"uneven batch of {len(jobs)}: radiance {worst_r:.2e}, Jacobian {worst_j:.2e}")
+
+
+def _by_one_block_and_as_chosen(ctx, kt, cia, jobs):
+    """The batch by 8 warps an item in order, and by a context that chooses."""
+    outs = []
+    for c, fixed in ((ctx, True), (cirsradg.Context(0), False)):
+        c.set_ktables(kt)
+        c.set_cia(cia)
+        if fixed:
+            c.set_tile(8)
+            c.set_schedule(0, 0)
+        try:
+            outs.append(c.cirsrtfg_wave_batch(jobs))
+        finally:
+            if fixed:
+                c.set_tile(0)
+    return outs
+
+
+# one item on a cluster of 8, 4 and 2 blocks of 16 warps, on one of 16, a pair of 8 and one of 8
+@pytest.mark.parametrize("nwave", [1, 9, 10, 18, 19, 37, 38, 74, 75, 148, 149, 222, 223])
+@pytest.mark.parametrize("nlayer,ng", [(2, 20), (23, 20), (40, 16)])
+def test_blocks_that_share_an_item_give_the_same_bits(ctx, nwave, nlayer, ng):
+    kt, cia = synth.make_ktables([synth.CH4, synth.C2H6], np_=6, nt=5, ng=ng, nbin=256, seed=ng), synth.make_cia(ng)
+    job = synth.make_job(kt, [synth.CH4, synth.C2H6], nlayer=nlayer, seed=nwave, nwave=nwave)
+    _same(*_by_one_block_and_as_chosen(ctx, kt, cia, [job]))
+
+
+# items below and from two a block on: in order, and pulled longest spectrum first
+@pytest.mark.parametrize("nwave", [60, 150, 450])
+def test_chosen_schedule_of_uneven_spectra_gives_the_same_bits(ctx, nwave):
+    kt, cia = synth.make_ktables([synth.CH4, synth.C2H6], np_=6, nt=5, ng=20, nbin=512, seed=3), synth.make_cia(3)
+    jobs = [synth.make_job(kt, [synth.CH4, synth.C2H6][:1 + k % 2], nlayer=n, seed=k, nwave=nwave)
+            for k, n in enumerate([5, 17, 9])]
+    _same(*_by_one_block_and_as_chosen(ctx, kt, cia, jobs))
+
+
+def test_autotune_of_a_small_batch_keeps_the_chosen_form(ctx):
+    """Few items: the form a context chooses by itself is among the candidates."""
+    kt, cia = synth.make_ktables([synth.CH4], np_=6, nt=5, ng=20, nbin=64, seed=5), synth.make_cia(5)
+    job = synth.make_job(kt, [synth.CH4], nlayer=40, seed=5, nwave=3)
+    one, = _by_one_block_and_as_chosen(ctx, kt, cia, [job])[:1]
+    c = cirsradg.Context(0)
+    c.set_ktables(kt)
+    c.set_cia(cia)
+    c.prepare([job])
+    tune = c.autotune()
+    assert tune["candidates"] >= 10 and tune["warps"] in (2, 4, 8, 16)
+    c.launch()
+    _same(c.fetch(), one)
