@@ -1288,7 +1288,8 @@ int apply_schedule(rtb_context* c) {
     // round trip costs more than it evens out.  14 spectra, 7000 items of 444
     // blocks: 4.20 ms static, 3.82 ms; 5 spectra, 1000 items: 296 and 264 us; one
     // spectrum of 515 items: 274 and 288 us
-    const bool dynamic = c->sched >= 1 || (c->sched < 0 && B.nitems >= 2 * (int64_t)c->grid);
+    // (never by a cluster, whose blocks have to take the same item)
+    const bool dynamic = B.cluster == 1 && (c->sched >= 1 || (c->sched < 0 && B.nitems >= 2 * (int64_t)c->grid));
     B.work_next = dynamic ? (unsigned long long*)((char*)c->d_diag.p + 48) : nullptr;
     B.item_order = c->sched < 0 && dynamic ? c->order_first : nullptr;
     if (c->sched == 2) {
