@@ -142,6 +142,13 @@ __device__ __forceinline__ unsigned bf16_pair(float lo, float hi) {
     return r;
 }
 
+// volatile: converted where it stands, not again at each use
+__device__ __forceinline__ double to_f64(float x) {
+    double d;
+    asm volatile("cvt.f64.f32 %0, %1;" : "=d"(d) : "f"(x));
+    return d;
+}
+
 struct PassSm {
     double* colp;     // [kNw][kKc] per-warp column partials
     double* wch;      // [kKc] Se^-1 (dy + K v) of the chunk
@@ -160,11 +167,12 @@ struct PassSm {
 // hi/lo for the tensor-core product N += K~ K~^T.  v and out hold kNp
 // entries (zero beyond nx).  Returns false if an mbarrier wait gave up.
 //
-// The conversions of K to FP64 (16 a cycle and SM, each element twice) and two
+// The conversions of K to FP64 (16 a cycle and SM, each element once) and two
 // barriers a chunk bound it; nothing waits for memory between the barriers: K, y
 // and Se^-1 of the next chunk are read while this one is worked on, and Se^-1/2
-// is formed once per wavenumber.  124 x 2000: about 60 us a pass, where loads
-// at the chunk's own time and a root per element took 100 us.
+// is formed once per wavenumber.  124 x 2000: 37 us a pass, 71 with the
+// tensor-core product, where loads at the chunk's own time and a root per element
+// took 100 us.
 template <bool kTc>
 __device__ bool k_pass(const NewtonDev& R, const double* v, bool with_dy, double* out, const PassSm& P) {
     const int nx = R.nx, ny = R.ny;
@@ -174,6 +182,7 @@ __device__ bool k_pass(const NewtonDev& R, const double* v, bool with_dy, double
 #pragma unroll
     for (int r = 0; r < 4; ++r) vr[r] = v[rb + 32 * r];
     float x[4][8], xn[4][8];
+    double xd[4][8];
     auto load = [&](int c) {
         const int nu0 = c * kKc + 8 * g8;
 #pragma unroll
@@ -208,7 +217,10 @@ __device__ bool k_pass(const NewtonDev& R, const double* v, bool with_dy, double
 #pragma unroll
         for (int r = 0; r < 4; ++r)
 #pragma unroll
-            for (int e = 0; e < 8; ++e) x[r][e] = xn[r][e];
+            for (int e = 0; e < 8; ++e) {
+                x[r][e] = xn[r][e];
+                xd[r][e] = to_f64(x[r][e]);
+            }
         if (c + 1 < nchunk) load(c + 1);
         // column partials over this thread's 4 rows, then over the warp's 4 row
         // groups: each exchange keeps half of the columns, so lane l ends with two
@@ -217,7 +229,7 @@ __device__ bool k_pass(const NewtonDev& R, const double* v, bool with_dy, double
         for (int e = 0; e < 8; ++e) {
             double s = 0.0;
 #pragma unroll
-            for (int r = 0; r < 4; ++r) s = fma((double)x[r][e], vr[r], s);
+            for (int r = 0; r < 4; ++r) s = fma(xd[r][e], vr[r], s);
             cp[e] = s;
         }
         {
@@ -291,7 +303,7 @@ __device__ bool k_pass(const NewtonDev& R, const double* v, bool with_dy, double
         for (int r = 0; r < 4; ++r) {
             double a = acc[r];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) a = fma((double)x[r][e], P.wch[8 * g8 + e], a);
+            for (int e = 0; e < 8; ++e) a = fma(xd[r][e], P.wch[8 * g8 + e], a);
             acc[r] = a;
         }
     }
@@ -317,10 +329,19 @@ __device__ bool k_pass(const NewtonDev& R, const double* v, bool with_dy, double
 }
 
 // C (nx x nx, row-major FP64) = N + Sa^-1 from the tensor-memory accumulator:
-// warp w reads lanes 32 (w & 3).. and columns 64 (w >> 2)..
+// warp w reads lanes 32 (w & 3).. and columns 64 (w >> 2)..  Sa^-1 is copied
+// to C first, every element in flight at once: read where a row is added, a row's
+// lanes lying nx apart, it took 15000 cycles (nx = 42), now 6300.
 __device__ void c_from_tmem(const NewtonDev& R, uint32_t tmem, double* C) {
     const int nx = R.nx, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int row = 32 * (warp & 3) + lane, c0 = 64 * (warp >> 2);
+    for (int i = warp; i < nx; i += kNw)
+        for (int j = lane; j < nx; j += 32)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(C + i * c_ld(nx) + j)),
+                         "l"(R.sai + i * nx + j)
+                         : "memory");
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
     tc_fence_after();
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -330,7 +351,7 @@ __device__ void c_from_tmem(const NewtonDev& R, uint32_t tmem, double* C) {
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
                 const int col = c0 + 16 * q + i;
-                if (col < nx) C[row * c_ld(nx) + col] = (double)v[i] + R.sai[row * nx + col];
+                if (col < nx) C[row * c_ld(nx) + col] += (double)v[i];
             }
         }
     }
@@ -390,8 +411,8 @@ __device__ void hessian_f64(const NewtonDev& R, char* sm, double* C) {
 // The chain of n reciprocal roots bounds it: one warp runs a panel's 16 x 16
 // diagonal block on shuffles without a barrier, then every row below goes on its
 // own thread, then the 16 x 16 thread grid updates the rest from registers.  One
-// reciprocal root per column instead of a root and divisions: n = 124 in 63 us
-// with those, column by column with three barriers each 240 us.
+// reciprocal root per column instead of a root and divisions: n = 124 in 46 us,
+// 63 with those, 240 column by column with three barriers each.
 constexpr int kPanel = 16;
 __device__ bool factor_ldlt(double* C, int n, int ld, double* rd) {
     const int tid = threadIdx.x, lane = tid & 31;
@@ -543,11 +564,16 @@ __device__ void apply_c_exact(const NewtonDev& R, const double* x, double* out, 
     const int nx = R.nx;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     k_pass<false>(R, x, false, out, P);
-    for (int i = warp; i < nx; i += kNw) {
-        double s = 0.0;
-        for (int j = lane; j < nx; j += 32) s = fma(R.sai[i * nx + j], x[j], s);
-        s = warp_sum(s);
-        if (lane == 0) out[i] += s;
+    for (int i0 = warp; i0 < nx; i0 += 4 * kNw) {    // four rows' reads in flight
+        double s[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int j = lane; j < nx; j += 32)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) s[r] = fma(R.sai[min(i0 + r * kNw, nx - 1) * nx + j], x[j], s[r]);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            s[r] = warp_sum(s[r]);
+            if (lane == 0 && i0 + r * kNw < nx) out[i0 + r * kNw] += s[r];
+        }
     }
     __syncthreads();
 }
@@ -679,7 +705,7 @@ phi_kernel(const PhiDev* __restrict__ rets, float* __restrict__ phi, float* __re
 // Ainv = A^-1 for SPD A (dinvertm.f jmod=2): Cholesky, then one identity
 // column per warp through the two triangular solves.  The columns of a matrix
 // are split over gridDim.y blocks, each with the (cheaper) factorisation of its
-// own: one 107 x 107 matrix takes 47 us over 14 blocks, where one block that
+// own: one 107 x 107 matrix takes 54 us over 14 blocks, where one block that
 // kept its columns in shared memory took 905 us.
 __global__ void __launch_bounds__(kNt, 1)
 spd_inverse_kernel(const double* __restrict__ A, double* __restrict__ Ainv, int n, int64_t stride,
