@@ -23,6 +23,7 @@ int fwd_tile_warps(bool t2, bool ext, int warps);
 size_t fwd_merge_table_bytes();
 void fwd_merge_table(int ng, void* table);
 int fwd_blocks_per_sm(int smem, bool t2, bool ext, int warps, int ng);
+int fwd_max_clusters(int smem, bool t2, bool ext, int warps, int ng, int size);   // resident at once
 cudaError_t launch_fwd(const BatchDev& B, int nsw, int ncol, int ngk, int nlmax, int npath, int grid, int warps,
                        cudaStream_t st);
 
@@ -195,7 +196,8 @@ struct rtb_context {
     rtb::DevBuf d_conv, d_convout;
     rtb::DevBuf d_layer;                  // rtb_layerg inputs, arguments and outputs
     std::vector<char> h_conv;
-    // fwd_blocks_per_sm by (shared bytes, t2, ext, tile, NG): a query of the driver per tile and call otherwise
+    // fwd_blocks_per_sm by (shared bytes, t2, ext, tile, NG), a query of the driver per tile and call otherwise;
+    // fwd_max_clusters with tile x (1 + cluster size)
     std::map<std::array<int, 5>, int> bpsm_known;
     size_t dbg_perm_n = 0, dbg_split_n = 0;
     rtb_fwd_stats stats{};

@@ -1097,6 +1097,28 @@ int fwd_blocks_per_sm(int smem, bool t2, bool ext, int warps, int ng) {
     return n;
 }
 
+int fwd_max_clusters(int smem, bool t2, bool ext, int warps, int ng, int size) {
+    const int w = fwd_tile_warps(t2, ext, warps);
+    const FwdKern k = fwd_instance(t2, ext, w, ng, false);
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = size;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(size);
+    cfg.blockDim = dim3(w * 32);
+    cfg.dynamicSmemBytes = smem;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return n;
+}
+
 cudaError_t launch_fwd(const BatchDev& B, int nsw, int ncol, int ngk, int nlmax, int npath, int grid, int warps,
                        cudaStream_t st) {
     const int w = fwd_tile_warps(B.t2, B.ext, warps);

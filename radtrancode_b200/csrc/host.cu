@@ -1259,6 +1259,18 @@ void drop_graph(rtb_context* c) {
     c->graph = nullptr;
 }
 
+// clusters of `size` blocks of the wide tile that the device runs at once
+int max_clusters(rtb_context* c, int size) {
+    const bool t2 = c->B.t2, ext = c->B.ext;
+    const int smem = fwd_smem_bytes(c->ng, c->nsw_max, c->ncol_max, c->ngk_max, c->nlmax_max, c->npath_max, kTileWide);
+    const std::array<int, 5> key = {smem, t2, ext, kTileWide * (1 + size), c->ng};
+    const auto known = c->bpsm_known.find(key);
+    if (known != c->bpsm_known.end()) return known->second;
+    const int n = fwd_max_clusters(smem, t2, ext, kTileWide, c->ng, size);
+    if (c->bpsm_known.size() < 256) c->bpsm_known[key] = n;
+    return n;
+}
+
 // grid, work counter and issue order of the resident batch from (sched, occ)
 int apply_schedule(rtb_context* c) {
     drop_graph(c);
@@ -1266,7 +1278,9 @@ int apply_schedule(rtb_context* c) {
     // With an SM or more for every item the layers of one run on twice the warps
     // (one wavenumber of 40 layers and 2 absorbers takes 89 us by 8 warps, 61 by
     // 16), and with two SMs or more on as many blocks of a cluster, up to 8, as
-    // there are SMs for and layers to share (30 us).  Beyond that, while two blocks
+    // there are SMs for and layers to share (30 us), so long as all clusters run at
+    // once: they do not cross GPCs, and 16 to 18 wavenumbers of 120 layers take 124 us
+    // by clusters of 8, of which 15 fit, 104 by 4.  Beyond that, while two blocks
     // of 8 warps an item are resident at once, on a pair of them: 80 layers, 16-point
     // tables, 149 wavenumbers 155 us by one block, 117 by two; 120 layers, 4
     // absorbers, 222 wavenumbers 592 and 545 us.
@@ -1280,7 +1294,9 @@ int apply_schedule(rtb_context* c) {
     c->grid = (int)std::max<int64_t>(grid, 1);
     B.cluster = 1;
     if (wide && c->sched < 1 && c->tile_eff == kTileWide)
-        while (B.cluster < 8 && 2 * B.cluster * B.nitems <= c->nsm && B.cluster < c->Lmax) B.cluster *= 2;
+        while (B.cluster < 8 && 2 * B.cluster * B.nitems <= c->nsm && B.cluster < c->Lmax &&
+               B.nitems <= max_clusters(c, 2 * B.cluster))
+            B.cluster *= 2;
     if (!c->tile && !wide && c->sched < 1 && c->occ <= 0 && 2 * (int64_t)B.nitems <= (int64_t)c->nsm * b)
         B.cluster = 2;
     // no schedule asked for: from two items a block on they are pulled from the
