@@ -45,7 +45,6 @@ constexpr int kKc = 64;                   // wavenumbers per chunk (one 128-byte
 constexpr int kTile = kNp * kKc * 2;      // bytes of one bf16 staging tile (16 KB)
 constexpr int kStage = 2 * kTile;         // hi + lo
 constexpr int kStaging = 2 * kStage + 1024;   // two stages, 1024-byte alignment slack
-constexpr int kPartLd = kNp + 1;         // row stride of a block's part of N, FP32 in shared memory
 constexpr int kStageF64 = 32 * kNp * 8 + 32 * 8;   // hessian_f64: 32 wavenumbers of K in FP64
 
 // C's rows lie an odd number of doubles apart, so a column's lie on different banks
@@ -53,7 +52,7 @@ __host__ __device__ constexpr int c_ld(int nx) { return nx | 1; }
 __host__ __device__ constexpr int cmax(int a, int b) { return a > b ? a : b; }
 // C (nx x nx FP64) aliased with the staging buffers of the pass over K
 __host__ __device__ constexpr int region_bytes(int nx) {
-    return (cmax(cmax(nx * c_ld(nx) * 8, kNp * kPartLd * 4), cmax(kStaging, kStageF64)) + 15) & ~15;
+    return (cmax(nx * c_ld(nx) * 8, cmax(kStaging, kStageF64)) + 15) & ~15;
 }
 // region + d, rhs, dx, res, 1 / D (kNp doubles each) + the pass's per-warp column
 // partials [kNw][kKc], the chunk's Se^-1 (dy + K d) [kKc], Se^-1/2 [2][kKc], 2 mbarriers and
@@ -150,38 +149,6 @@ __device__ __forceinline__ double to_f64(float x) {
     return d;
 }
 
-// ---------------------------------------------------------------- blocks of a cluster
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ uint32_t cluster_size() {
-    uint32_t n;
-    asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(n));
-    return n;
-}
-// all threads of the cluster; what they wrote to shared memory before is seen after
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
-// block `rank`'s word at this block's shared address
-__device__ __forceinline__ uint32_t at_rank(const void* p, int rank) {
-    uint32_t r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ float ld_cluster_f32(uint32_t a) {
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
-    return v;
-}
-__device__ __forceinline__ double ld_cluster_f64(uint32_t a) {
-    double v;
-    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
-    return v;
-}
-
 struct PassSm {
     double* colp;     // [kNw][kKc] per-warp column partials
     double* wch;      // [kKc] Se^-1 (dy + K v) of the chunk
@@ -189,7 +156,6 @@ struct PassSm {
     uint32_t stage0;  // shared address of the first staging stage (1024-aligned)
     uint32_t bar0;    // shared address of the two mbarriers
     uint32_t tmem;    // accumulator address in tensor memory
-    int rank, size;   // this block takes chunks rank, rank + size, ...
 };
 
 // One pass over K (nx x ny, FP32, row iv = dR/dx_iv) in chunks of kKc
@@ -199,9 +165,7 @@ struct PassSm {
 //   out(i) += sum_nu K(i, nu) w(nu)                           (FP64 accumulation)
 // and with kTc the chunk's K~ = Se^-1/2 K goes to shared memory as bf16
 // hi/lo for the tensor-core product N += K~ K~^T.  v and out hold kNp
-// entries (zero beyond nx).  Returns false if an mbarrier wait gave up.  The blocks
-// of a cluster share the chunks (each has one at least); out and the tensor-core
-// product are then each block's part.
+// entries (zero beyond nx).  Returns false if an mbarrier wait gave up.
 //
 // The conversions of K to FP64 (16 a cycle and SM, each element once) and two
 // barriers a chunk bound it; nothing waits for memory between the barriers: K, y
@@ -247,11 +211,9 @@ __device__ bool k_pass(const NewtonDev& R, const double* v, bool with_dy, double
     const int nchunk = (ny + kKc - 1) / kKc;
     bool ok = true;
     uint32_t phase[2] = {0u, 0u};
-    const int step = P.size, c_first = P.rank;
-    load(c_first);
-    load_y(c_first);
-    int it = 0;
-    for (int c = c_first; c < nchunk; c += step, ++it) {
+    load(0);
+    load_y(0);
+    for (int c = 0; c < nchunk; ++c) {
 #pragma unroll
         for (int r = 0; r < 4; ++r)
 #pragma unroll
@@ -259,7 +221,7 @@ __device__ bool k_pass(const NewtonDev& R, const double* v, bool with_dy, double
                 x[r][e] = xn[r][e];
                 xd[r][e] = to_f64(x[r][e]);
             }
-        if (c + step < nchunk) load(c + step);
+        if (c + 1 < nchunk) load(c + 1);
         // column partials over this thread's 4 rows, then over the warp's 4 row
         // groups: each exchange keeps half of the columns, so lane l ends with two
         double cp[8];
@@ -282,9 +244,9 @@ __device__ bool k_pass(const NewtonDev& R, const double* v, bool with_dy, double
                 P.colp[warp * kKc + 8 * g8 + (b3 ? 4 : 0) + (b4 ? 2 : 0) + e] = k2[e];
             }
         }
-        const int s = it & 1;
+        const int s = c & 1;
         if (kTc && tid < kKc) P.sc[s * kKc + tid] = (float)sqrt(se);
-        if (kTc && it >= 2) {   // stage s is free once the MMAs of the chunk before the last are complete
+        if (kTc && c >= 2) {   // stage s is free once the MMAs of chunk c - 2 are complete
             if (tid == 0 && !mbar_wait(P.bar0 + 8 * s, phase[s])) ok = false;
             phase[s] ^= 1u;
         }
@@ -295,7 +257,7 @@ __device__ bool k_pass(const NewtonDev& R, const double* v, bool with_dy, double
             for (int w8 = 0; w8 < kNw; ++w8) cs += P.colp[w8 * kKc + tid];
             P.wch[tid] = ((double)dy + cs) * se;
         }
-        if (c + step < nchunk) load_y(c + step);
+        if (c + 1 < nchunk) load_y(c + 1);
         if (kTc) {
             float sc[8];
 #pragma unroll
@@ -330,7 +292,7 @@ __device__ bool k_pass(const NewtonDev& R, const double* v, bool with_dy, double
 #pragma unroll
             for (int k = 0; k < kKc / 16; ++k) {
                 const uint64_t dh = sw128_desc(hi + 32 * k), dl = sw128_desc(lo + 32 * k);
-                umma_bf16(P.tmem, dh, dh, (it > 0 || k > 0) ? 1u : 0u);
+                umma_bf16(P.tmem, dh, dh, (c > 0 || k > 0) ? 1u : 0u);
                 umma_bf16(P.tmem, dh, dl, 1u);
                 umma_bf16(P.tmem, dl, dh, 1u);
             }
@@ -348,7 +310,7 @@ __device__ bool k_pass(const NewtonDev& R, const double* v, bool with_dy, double
     if (kTc && tid == 0) {
         // the last commit completes after every MMA of the pass; should it not
         // arrive in time, wait once more (bounded) before tensor memory is freed
-        const int sl = (it - 1) & 1;
+        const int sl = (nchunk - 1) & 1;
         if (!mbar_wait(P.bar0 + 8 * sl, phase[sl])) {
             ok = false;
             mbar_wait(P.bar0 + 8 * sl, phase[sl]);
@@ -370,13 +332,11 @@ __device__ bool k_pass(const NewtonDev& R, const double* v, bool with_dy, double
 // warp w reads lanes 32 (w & 3).. and columns 64 (w >> 2)..  Sa^-1 is copied
 // to C first, every element in flight at once: read where a row is added, a row's
 // lanes lying nx apart, it took 15000 cycles (nx = 42), now 6300.
-// Only the lower triangle, which is all that the factorisation reads.  The other
-// blocks of a cluster left their parts of N in FP32 at `part` of their shared memory.
-__device__ void c_from_tmem(const NewtonDev& R, uint32_t tmem, double* C, const float* part, int size) {
+__device__ void c_from_tmem(const NewtonDev& R, uint32_t tmem, double* C) {
     const int nx = R.nx, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int row = 32 * (warp & 3) + lane, c0 = 64 * (warp >> 2);
     for (int i = warp; i < nx; i += kNw)
-        for (int j = lane; j <= i; j += 32)
+        for (int j = lane; j < nx; j += 32)
             asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(C + i * c_ld(nx) + j)),
                          "l"(R.sai + i * nx + j)
                          : "memory");
@@ -385,51 +345,17 @@ __device__ void c_from_tmem(const NewtonDev& R, uint32_t tmem, double* C, const 
     tc_fence_after();
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-        const int col0 = c0 + 16 * q;
         float v[16];
-        tmem_ld16(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)col0, v);
-        if (row < nx && col0 <= row) {
-            double sum[16];
+        tmem_ld16(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(c0 + 16 * q), v);
+        if (row < nx) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) sum[i] = (double)v[i];
-            for (int r = 1; r < size; ++r) {
-                const uint32_t src = at_rank(part, r) + (uint32_t)(row * kPartLd + col0) * 4;
-#pragma unroll
-                for (int i = 0; i < 16; ++i) v[i] = ld_cluster_f32(src + 4 * i);
-#pragma unroll
-                for (int i = 0; i < 16; ++i) sum[i] += (double)v[i];
+            for (int i = 0; i < 16; ++i) {
+                const int col = c0 + 16 * q + i;
+                if (col < nx) C[row * c_ld(nx) + col] += (double)v[i];
             }
-#pragma unroll
-            for (int i = 0; i < 16; ++i)
-                if (col0 + i <= row) C[row * c_ld(nx) + col0 + i] += sum[i];
         }
     }
     tc_fence_before();
-    __syncthreads();
-}
-
-// this block's part of N to shared memory
-__device__ void part_from_tmem(uint32_t tmem, float* part) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int row = 32 * (warp & 3) + lane, c0 = 64 * (warp >> 2);
-    tc_fence_after();
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        float v[16];
-        tmem_ld16(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(c0 + 16 * q), v);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) part[row * kPartLd + c0 + 16 * q + i] = v[i];
-    }
-    tc_fence_before();
-}
-
-// out of the first block of a cluster += the others' in their order
-__device__ void sum_parts(double* out, int size) {
-    if (threadIdx.x < kNp) {
-        double s = out[threadIdx.x];
-        for (int r = 1; r < size; ++r) s += ld_cluster_f64(at_rank(out + threadIdx.x, r));
-        out[threadIdx.x] = s;
-    }
     __syncthreads();
 }
 
@@ -633,17 +559,11 @@ __device__ void ldlt_solve_shared(const double* L, int n, int ld, const double* 
     __syncwarp();
 }
 
-// out = (K^T Se^-1 K + Sa^-1) x, K applied in FP64 from FP32: one pass over K, the
-// result in the first block of a cluster
+// out = (K^T Se^-1 K + Sa^-1) x, K applied in FP64 from FP32: one pass over K
 __device__ void apply_c_exact(const NewtonDev& R, const double* x, double* out, const PassSm& P) {
     const int nx = R.nx;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     k_pass<false>(R, x, false, out, P);
-    if (P.size > 1) {
-        cluster_sync();
-        if (P.rank > 0) return;
-        sum_parts(out, P.size);
-    }
     for (int i0 = warp; i0 < nx; i0 += 4 * kNw) {    // four rows' reads in flight
         double s[4] = {0.0, 0.0, 0.0, 0.0};
         for (int j = lane; j < nx; j += 32)
@@ -658,20 +578,12 @@ __device__ void apply_c_exact(const NewtonDev& R, const double* x, double* out, 
     __syncthreads();
 }
 
-// A cluster of blocks shares a retrieval's passes over K: each takes every size-th
-// chunk, and the first block adds the parts, factors and solves.  Every block
-// reaches every cluster_sync: the flags that end a step early are read alike by all.
 template <int kHess>
 __global__ void __launch_bounds__(kNt, 1)
 newton_step_kernel(const NewtonDev* __restrict__ rets, int refine, unsigned* __restrict__ status,
                    double* __restrict__ resid) {
     extern __shared__ __align__(16) char smem[];
-    __shared__ float s_ok;
-    PassSm P;
-    P.rank = (int)cluster_rank();
-    P.size = (int)cluster_size();
-    const int ret = blockIdx.x / P.size;
-    const NewtonDev R = rets[ret];
+    const NewtonDev R = rets[blockIdx.x];
     const int nx = R.nx;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     double* C = (double*)smem;
@@ -679,6 +591,7 @@ newton_step_kernel(const NewtonDev* __restrict__ rets, int refine, unsigned* __r
     double* rhs = d + kNp;
     double* dx = rhs + kNp;
     double* res = dx + kNp;
+    PassSm P;
     double* rd = res + kNp;
     P.colp = rd + kNp;
     P.wch = P.colp + kNw * kKc;
@@ -707,50 +620,30 @@ newton_step_kernel(const NewtonDev* __restrict__ rets, int refine, unsigned* __r
     if (kHess == 0) {
         tc_fence_after();
         P.tmem = *tslot;
-        bool ok = k_pass<true>(R, d, true, rhs, P);   // N in tensor memory, rhs = K^T Se^-1 (y - yn + K d)
-        if (P.size > 1) {
-            if (P.rank > 0 && ok) part_from_tmem(P.tmem, (float*)smem);
-            if (tid == 0) s_ok = ok ? 1.0f : 0.0f;
-            cluster_sync();
-            for (int r = 0; r < P.size; ++r) ok = ok && ld_cluster_f32(at_rank(&s_ok, r)) != 0.0f;
-        }
-        if (P.rank == 0 && ok) {
-            if (P.size > 1) sum_parts(rhs, P.size);
-            c_from_tmem(R, P.tmem, C, (const float*)smem, P.size);
-        }
+        const bool ok = k_pass<true>(R, d, true, rhs, P);   // N in tensor memory, rhs = K^T Se^-1 (y - yn + K d)
+        if (ok) c_from_tmem(R, P.tmem, C);
         if (warp == 0) {
             tc_fence_after();
             asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(P.tmem), "r"(kNp));
         }
         if (!ok) {
-            if (P.size > 1) cluster_sync();
-            if (P.rank == 0 && tid == 0 && status) status[ret] = kNtTimeout;
+            if (tid == 0 && status) status[blockIdx.x] = kNtTimeout;
             return;
         }
     } else {
         hessian_f64(R, smem, C);
         k_pass<false>(R, d, true, rhs, P);
     }
+    const bool bad = factor_ldlt(C, nx, c_ld(nx), rd);
+    if (tid == 0 && status) status[blockIdx.x] = bad ? kNtNonPd : 0u;
     // padded entries stay 0: the passes over K read all kNp of them
-    if (P.rank == 0) {
-        const bool bad = factor_ldlt(C, nx, c_ld(nx), rd);
-        if (tid == 0 && status) status[ret] = bad ? kNtNonPd : 0u;
-        for (int i = tid; i < kNp; i += kNt) dx[i] = i < nx ? rhs[i] : 0.0;
-        __syncthreads();
-        if (warp == 0) ldlt_solve_shared(C, nx, c_ld(nx), rd, dx);
-        __syncthreads();
-    }
+    for (int i = tid; i < kNp; i += kNt) dx[i] = i < nx ? rhs[i] : 0.0;
+    __syncthreads();
+    if (warp == 0) ldlt_solve_shared(C, nx, c_ld(nx), rd, dx);
+    __syncthreads();
     const int nsteps = refine + (resid ? 1 : 0);
     for (int it = 0; it < nsteps; ++it) {
-        if (P.size > 1) {
-            cluster_sync();                // the first block's dx; it is done with the parts before
-            if (P.rank > 0) {
-                if (tid < kNp) dx[tid] = ld_cluster_f64(at_rank(dx + tid, 0));
-                __syncthreads();
-            }
-        }
         apply_c_exact(R, dx, res, P);
-        if (P.rank > 0) continue;
         for (int i = tid; i < nx; i += kNt) res[i] = rhs[i] - res[i];
         __syncthreads();
         if (it == refine) {            // residual of the final dx (no further update)
@@ -762,7 +655,7 @@ newton_step_kernel(const NewtonDev* __restrict__ rets, int refine, unsigned* __r
                 }
                 rr = warp_sum(rr);
                 bb = warp_sum(bb);
-                if (lane == 0) resid[ret] = bb > 0.0 ? sqrt(rr / bb) : sqrt(rr);
+                if (lane == 0) resid[blockIdx.x] = bb > 0.0 ? sqrt(rr / bb) : sqrt(rr);
             }
             break;
         }
@@ -771,8 +664,6 @@ newton_step_kernel(const NewtonDev* __restrict__ rets, int refine, unsigned* __r
         for (int i = tid; i < nx; i += kNt) dx[i] += res[i];
         __syncthreads();
     }
-    if (P.size > 1) cluster_sync();        // the first block has read the others' shared memory
-    if (P.rank > 0) return;
     for (int i = tid; i < nx; i += kNt) R.x_out[i] = R.xa[i] + (float)dx[i];   // calcnextxn.f:104
 }
 
@@ -843,33 +734,21 @@ spd_inverse_kernel(const double* __restrict__ A, double* __restrict__ Ainv, int 
 
 }  // namespace
 
-cudaError_t launch_newton_step(const NewtonDev* d_ret, int nret, int ny_least, int hessian, int refine,
-                               unsigned* d_status, double* d_resid, cudaStream_t st) {
+cudaError_t launch_newton_step(const NewtonDev* d_ret, int nret, int hessian, int refine, unsigned* d_status,
+                               double* d_resid, cudaStream_t st) {
     if (nret <= 0) return cudaSuccess;
     const int smem = newton_smem(kNp);
-    // Blocks per retrieval: two where both have an SM and two chunks of K, four where
-    // the chip holds that many clusters of four (its GPCs of 16 to 20 SMs: 32) and each
-    // block has four chunks.  18 retrievals of 124 x 2000: 232 us by one block each, 174
-    // by two, 152 by four, 320 by eight, which do not fit at once; of 124 x 1030 180,
-    // 148, 142 and 312; 8 of 124 x 520 131, 125 and 129; 4 of 42 x 200 58, 56 and 55.
-    const int nchunk = (ny_least + kKc - 1) / kKc;
-    int size = 1;
-    if (hessian == 0 && nret <= 74 && nchunk >= 4) size = nret <= 32 && nchunk >= 16 ? 4 : 2;
-    const auto kern = hessian == 0 ? newton_step_kernel<0> : newton_step_kernel<1>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = size;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(nret * size);
-    cfg.blockDim = dim3(kNt);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, d_ret, refine, d_status, d_resid);
+    cudaError_t e;
+    if (hessian == 0) {
+        e = cudaFuncSetAttribute(newton_step_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return e;
+        newton_step_kernel<0><<<nret, kNt, smem, st>>>(d_ret, refine, d_status, d_resid);
+    } else {
+        e = cudaFuncSetAttribute(newton_step_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return e;
+        newton_step_kernel<1><<<nret, kNt, smem, st>>>(d_ret, refine, d_status, d_resid);
+    }
+    return cudaGetLastError();
 }
 
 cudaError_t launch_phi(const PhiDev* d_ret, int nret, float* d_phi, float* d_chisq, cudaStream_t st) {

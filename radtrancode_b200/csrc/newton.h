@@ -41,9 +41,8 @@ struct PhiDev {
 // 1 = K^T Se^-1 K in FP64 on the CUDA cores (the all-FP64 solve).
 // resid (may be null): per retrieval ||rhs - C dx|| / ||rhs|| after the
 // last refinement step, with C applied exactly in FP64.
-// ny_least: the fewest measurements of any of the retrievals.
-cudaError_t launch_newton_step(const NewtonDev* d_ret, int nret, int ny_least, int hessian, int refine,
-                               unsigned* d_status, double* d_resid, cudaStream_t st);
+cudaError_t launch_newton_step(const NewtonDev* d_ret, int nret, int hessian, int refine, unsigned* d_status,
+                               double* d_resid, cudaStream_t st);
 // phi (REAL, as the reference function) and chisq per retrieval
 cudaError_t launch_phi(const PhiDev* d_ret, int nret, float* d_phi, float* d_chisq, cudaStream_t st);
 // Sa^-1 from Sa (FP64 Cholesky inverse, dinvertm.f jmod=2) for nret

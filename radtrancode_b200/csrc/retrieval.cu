@@ -728,12 +728,10 @@ struct Engine {
             d.x_out = X(*s, 3);
             desc.push_back(d);
         }
-        int ny_least = desc.empty() ? 0 : desc[0].ny;
-        for (const NewtonDev& d : desc) ny_least = std::min(ny_least, (int)d.ny);
         CUDA_TRY(c, h2d(nt_desc, desc, st));
         CUDA_TRY(c, small.ensure(12 * v.size() + 64));
-        CUDA_TRY(c, launch_newton_step((const NewtonDev*)nt_desc.p, (int)v.size(), ny_least, c->newton_hess,
-                                       c->newton_refine, (unsigned*)small.p, nullptr, st));
+        CUDA_TRY(c, launch_newton_step((const NewtonDev*)nt_desc.p, (int)v.size(), c->newton_hess, c->newton_refine,
+                                       (unsigned*)small.p, nullptr, st));
         std::vector<float> xs((size_t)rows * kXRow);
         std::vector<unsigned> sts(v.size());
         CUDA_TRY(c, cudaMemcpyAsync(xs.data(), xarea.p, xs.size() * 4, cudaMemcpyDeviceToHost, st));
@@ -1001,7 +999,7 @@ int rtb_newton_step_batch(rtb_context* c, int nret, int nx, int ny, const float*
     unsigned* status = (unsigned*)c->d_ntsmall.p;
     double* dres = (double*)((char*)c->d_ntsmall.p + ((4 * (size_t)nret + 15) & ~(size_t)15));
     CUDA_TRY(c, cudaEventRecord(c->ev0, st));
-    CUDA_TRY(c, launch_newton_step((const NewtonDev*)c->d_ntdesc.p, nret, ny, c->newton_hess, c->newton_refine, status,
+    CUDA_TRY(c, launch_newton_step((const NewtonDev*)c->d_ntdesc.p, nret, c->newton_hess, c->newton_refine, status,
                                    resid ? dres : nullptr, st));
     CUDA_TRY(c, cudaEventRecord(c->ev1, st));
     CUDA_TRY(c, cudaMemcpy2DAsync(x_out, nx * 4, F + o_xo, nxa * 4, nx * 4, nret, cudaMemcpyDeviceToHost, st));
