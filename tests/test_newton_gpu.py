@@ -379,3 +379,37 @@ def test_retrieval_of_dust_scales(ctx, oracle):
     sig = np.sqrt(np.diag(case.sa)).astype(np.float32)
     assert np.all(np.abs(g["x"] - ref["x"]) <= 1e-3 * sig)
     assert abs(g["phi"] - ref["phi"]) <= 1e-3 * ref["phi"]
+
+
+def _random_inputs(nret, nx, ny):
+    """A well-conditioned problem: K ~ N(0, 1), Se^-1 in 0.5..2, Sa^-1 = 4 I + a tenth of a random SPD matrix."""
+    rng = np.random.default_rng(1000 * nx + ny + nret)
+    kk = rng.standard_normal((nret, nx, ny)).astype(np.float32)
+    sei = rng.uniform(0.5, 2.0, (nret, ny))
+    b = rng.standard_normal((nret, nx, nx))
+    sai = 4.0 * np.eye(nx) + 0.1 * b @ b.transpose(0, 2, 1) / nx
+    xa, xn = (rng.standard_normal((nret, nx)).astype(np.float32) for _ in range(2))
+    y, yn = (rng.standard_normal((nret, ny)).astype(np.float32) for _ in range(2))
+    return kk, sei, sai, xa, xn, y, yn
+
+
+# one block a matrix, and its columns over several; panels of 16 and their remainders
+@pytest.mark.parametrize("nret", [1, 10, 80])
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 31, 33, 64, 112, 113, 127, 128])
+def test_spd_inverse_at_panel_edges(ctx, nret, n):
+    _, _, a, *_ = _random_inputs(nret, n, 1)
+    inv, nonpd = ctx.spd_inverse_batch(a)
+    assert not nonpd.any()
+    ref = np.linalg.inv(a)
+    assert np.max(np.abs(inv - ref)) <= 1e-10 * np.max(np.abs(ref))
+
+
+# k groups of a block and chunks of 16 with remainders, both ways round
+@pytest.mark.parametrize("nx,ny", [(1, 2), (3, 5), (16, 17), (17, 63), (33, 130), (107, 111), (128, 129)])
+def test_gain_products_at_chunk_edges(ctx, oracle, nx, ny):
+    kk, sei, sai, *_ = _random_inputs(1, nx, ny)
+    dd, aa, nonpd = ctx.calc_gain_matrix(kk[0], sai[0], sei[0])
+    dd_r, aa_r = oracle.gain_matrix(kk[0], sei[0], sai[0])
+    assert nonpd == 0
+    assert np.max(np.abs(dd - dd_r)) <= 1e-9 * np.max(np.abs(dd_r))
+    assert np.max(np.abs(aa - aa_r)) <= 1e-9 * np.max(np.abs(aa_r))
