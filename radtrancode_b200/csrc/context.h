@@ -16,8 +16,8 @@
 
 namespace rtb {
 int fwd_smem_bytes(int ng, int nsw, int ncol, int ngk, int nlmax, int npath, int warps);
-// warps per CTA a launch uses for a requested tile (tiles other than kWarps
-// exist for the usual instance only), and the blocks per SM it can hold
+// warps per CTA a launch uses for a requested tile (2 and 4 exist for the usual
+// instance only), and the blocks per SM it can hold
 int fwd_tile_warps(bool t2, bool ext, int warps);
 // the overlap merge's per-level, per-lane table of an NG (MergeLane)
 size_t fwd_merge_table_bytes();

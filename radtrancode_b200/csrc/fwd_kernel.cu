@@ -2,8 +2,9 @@
 // thermal-emission path (radtran/cirsradg/cirsradg_wave.f, IMOD 0/1/3) fused
 // with map2pro/map2xvec (radtran/cirsradg/map2pro.f, map2xvec.f).
 //
-// One CTA (8 warps) owns one (spectrum, wavenumber) work item at a time and
-// loops over items grid-stride (persistent grid, one scratch slot per CTA).
+// One CTA (8 warps; 16, or several CTAs of a cluster, where SMs would be idle) owns
+// one (spectrum, wavenumber) work item at a time and loops over items, grid-stride or
+// pulled from a counter (persistent grid, one scratch slot per CTA or cluster).
 //   A  per layer (one warp each): k-table interpolation of every gas
 //      (get_kg.f:306-378), continuum optical depth and its derivatives
 //      (nciacon.f, dust, Rayleigh: cirsradg_wave.f:510-691) and the random
@@ -632,7 +633,8 @@ __device__ __forceinline__ void cluster_sync() {
 // ext: some spectrum takes the para-H2 CIA (flagh2p = 1), an IMOD 18 path or
 // iform = 3.  Template arguments, so that the usual kernel carries no trace
 // of either.  WARPS: warps per CTA, the layers of one (spectrum, wavenumber)
-// item worked on at once -- the tile shape the autotuner chooses.  The
+// item worked on at once -- the tile shape the autotuner chooses.  CL = 2: two CTAs
+// of a cluster share an item's layers (the wide tile: B.cluster of them).  The
 // residency bound keeps 24 warps per SM at 80 registers: the passes wait on
 // shuffles and fixed-latency chains, and 16 warps at 128 registers took 4.28 ms
 // where 24 take 4.04 ms (120 layers, 4 absorbers, 2000 wavenumbers).  NGC > 0:
@@ -1057,9 +1059,9 @@ using FwdKern = void (*)(BatchDev, int, int, int, int, int);
 // warps, and NG = 20 as a constant, exist for the usual instance only (one
 // temperature grid, no extended options).  Up to 256 elements a pass are
 // sorted in registers, more are merged in shared memory: one spectrum of
-// 16-point tables (80 layers, 150 wavenumbers, 2 absorbers) takes 0.22 ms by
-// the first and 0.27 ms by the second, one of 20-point tables (120 layers, 2000
-// wavenumbers, 4 absorbers) 3.68 and 3.45 ms.
+// 16-point tables (80 layers, 150 wavenumbers, 2 absorbers, a block an item) takes
+// 0.22 ms by the first and 0.27 ms by the second, one of 20-point tables (120
+// layers, 2000 wavenumbers, 4 absorbers) 3.68 and 3.45 ms.
 constexpr int kNgConst = 20;
 template <bool t2, bool ext, int WARPS, int CL = 1>
 FwdKern fwd_by_ng(int ng) {
