@@ -223,20 +223,17 @@ __device__ __forceinline__ void interp_lin(const float* t, const KgPos& L, int g
 
 // get_kg for a wavenumber between two table points (get_kg.f:380-438):
 // 2 NG linearly interpolated values, weighted (1 - w2) delg and w2 delg,
-// rank-rebinned by rankk on lane 0.  scr: per-warp shared scratch of at least
-// 8 * kMaxNg floats + 2 * kMaxNg shorts.  Called by the whole warp.
+// rank-rebinned by rankk on lane 0.  scr: per-warp shared scratch (rankk_off).
+// Called by the whole warp.
 template <bool t2>
 __device__ void get_kg_lane_nc(const BatchDev& B, int64_t slice, float w1, float w2, const KgPos& L, int lane,
                                float* scr,
                                float& k, float& dk) {
     const int ng = B.ng;
-    float* cont = scr;
-    float* dcont = scr + 2 * kMaxNg;
-    float* fac = scr + 4 * kMaxNg;
-    float* tmp = scr + 6 * kMaxNg;                  // 2 ng + 1 entries
-    float* kg = scr + 8 * kMaxNg + 2;
-    float* dkg = kg + kMaxNg;
-    unsigned short* ico = (unsigned short*)(dkg + kMaxNg);
+    const RankkOff o = rankk_off(ng);
+    float *cont = scr + o.cont, *dcont = scr + o.dcont, *fac = scr + o.fac, *tmp = scr + o.tmp;
+    float *kg = scr + o.kg, *dkg = scr + o.dkg;
+    unsigned short* ico = (unsigned short*)(scr + o.ico);
     k = 0.0f;
     dk = 0.0f;
     if (slice < 0) return;

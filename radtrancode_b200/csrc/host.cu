@@ -1009,7 +1009,8 @@ static void longest_first(const rtb_context* c, std::vector<int>& order) {
 int prepare_ex(rtb_context* c, int nspec, const rtb_atm* atms, const OutPlace* place) {
     if (!c || nspec <= 0 || !atms) return fail(c, RTB_ERR_ARG, "bad batch arguments");
     if (c->ntab <= 0) return fail(c, RTB_ERR_NOTABLE, "no k-tables loaded");
-    if (c->ng > 22 || c->ng < 2) return fail(c, RTB_ERR_UNSUPPORTED, "NG=%d outside the device range 2..22", c->ng);
+    if (c->ng > kNgMax || c->ng < kNgMin)
+        return fail(c, RTB_ERR_UNSUPPORTED, "NG=%d outside the device range %d..%d", c->ng, kNgMin, kNgMax);
     CUDA_TRY(c, cudaSetDevice(c->device));
     c->prepared = 0;
     // instrument convolution of each spectrum's outputs (cirsrtfg_wave.f:448-516)

@@ -263,6 +263,22 @@ __host__ __device__ constexpr int pass_scratch_bytes(int ng, int ncol, int ngk) 
     return (pass_kg_offset(ng) + 8 * ngk * ng + 4 * ncol * ng + 15) & ~15;
 }
 
+// The same scratch as the work arrays of rankk, at offsets in 32-bit words: value,
+// derivative and weight of its 2 NG elements, 2 NG + 1 words of work, k and dk/dT of
+// the NG bins, the elements' order in 16 bits.
+struct RankkOff {
+    int cont, dcont, fac, tmp, kg, dkg, ico, bytes;
+};
+__host__ __device__ constexpr RankkOff rankk_off(int ng) {
+    return {0, 2 * ng, 4 * ng, 6 * ng, 8 * ng + 1, 9 * ng + 1, 10 * ng + 1, 4 * (10 * ng + 1) + 2 * 2 * ng};
+}
+constexpr bool rankk_fits() {
+    for (int ng = kNgMin; ng <= kNgMax; ++ng)
+        if (rankk_off(ng).bytes > pass_scratch_bytes(ng, 0, 0)) return false;
+    return true;
+}
+static_assert(rankk_fits(), "rankk's work arrays lie in one warp's scratch at every NG");
+
 template <int N>
 struct Const {              // a compile-time number as an argument
     static constexpr int value = N;

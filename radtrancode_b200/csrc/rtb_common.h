@@ -10,6 +10,7 @@
 namespace rtb {
 
 constexpr int kMaxNg = 32;        // one lane per g-ordinate
+constexpr int kNgMin = 2, kNgMax = 22;   // the NG that a forward call takes
 constexpr int kMaxCols = 8;       // tracked gradient columns in the overlap (active gases + T)
 constexpr int kMaxSw = 8;         // active Jacobian columns (isw) per spectrum
 constexpr int kMaxGasDev = 30;    // MAXGAS

@@ -274,6 +274,34 @@ def test_noncoincident_wavenumbers(ctx, oracle, shift):
     assert not np.array_equal(c0, c)
 
 
+@pytest.mark.parametrize("tile", [0, 8])     # 0: the wide tile, these calls having few wavenumbers
+@pytest.mark.parametrize("nabs", [1, 2, 4])
+@pytest.mark.parametrize("ng", [2, 5, 6, 8, 9])
+def test_noncoincident_wavenumbers_at_small_ng(ctx, oracle, ng, nabs, tile):
+    """rankk's work arrays in a warp's scratch, which shrinks with NG and the
+    number of absorbers, while every warp of a block is in it: as
+    test_noncoincident_wavenumbers, bins of every pass included."""
+    gases = synth.ABSORBERS_C2[:nabs]
+    kt, cia = synth.make_ktables(gases, np_=6, nt=5, ng=ng, nbin=16, seed=100 + ng), synth.make_cia(ng)
+    j = _off_grid(synth.make_job(kt, gases, nlayer=19, seed=ng, nwave=12, vmr_perturb=0.3), kt, 0.37)
+    ctx.set_ktables(kt)
+    ctx.set_cia(cia)
+    ctx.set_debug(True)
+    ctx.set_tile(tile)
+    try:
+        c, g, _ = ctx.cirsrtfg_wave(j)
+        perm, split = ctx.debug_bins(j)
+    finally:
+        ctx.set_debug(False)
+        ctx.set_tile(0)
+    c64, g64, _ = oracle.cirsrtfg_wave(kt, cia, j, oracle.ORC_FP64)
+    assert rad_err(c, c64) <= RAD_TOL
+    assert jac_err(g, g64, j.nv) <= JAC_TOL
+    _, (operm, osplit, _) = oracle.cirsrtfg_wave(kt, cia, j, oracle.ORC_MIXED, debug=True)
+    assert np.array_equal(assignment(perm, split, ng), assignment(operm, osplit, ng))
+    assert np.array_equal(split, osplit)
+
+
 def test_cirsradg_wave_compat_matches_cirsrtfg_wave(ctx):
     """The per-wavenumber form (cirsradg_wave's output and doutputdq): its
     radiance is the whole-spectrum call's bit for bit, and map2pro + map2xvec
