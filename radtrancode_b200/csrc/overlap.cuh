@@ -245,7 +245,8 @@ __device__ __forceinline__ void warp_sort(float (&x)[E], int lane) {
 
 // Scratch of one warp's pass, in sorted order: the elements' records and the
 // FP64 prefix of the weights over each lane's chunk (the positions from NG * NG
-// on are pads).  Both also take the merge's runs, and gd the heapsort's words.
+// on are pads).  Both also take the merge's runs, and gd the heapsort's words and
+// the sequential walk's new columns.
 struct PassScratch {
     double* gd;        // [32 * chunk]
     uint2* rec;        // [32 * chunk + 1]: {key * weight, word}; the last one an empty element
@@ -272,12 +273,12 @@ struct RankkOff {
 __host__ __device__ constexpr RankkOff rankk_off(int ng) {
     return {0, 2 * ng, 4 * ng, 6 * ng, 8 * ng + 1, 9 * ng + 1, 10 * ng + 1, 4 * (10 * ng + 1) + 2 * 2 * ng};
 }
-constexpr bool rankk_fits() {
+constexpr bool scratch_fits() {
     for (int ng = kNgMin; ng <= kNgMax; ++ng)
-        if (rankk_off(ng).bytes > pass_scratch_bytes(ng, 0, 0)) return false;
+        if (rankk_off(ng).bytes > pass_scratch_bytes(ng, 0, 0) || 4 * kMaxCols * ng > pass_gd_bytes(ng)) return false;
     return true;
 }
-static_assert(rankk_fits(), "rankk's work arrays lie in one warp's scratch at every NG");
+static_assert(scratch_fits(), "at every NG rankk's arrays lie in one warp's scratch, the sequential walk's columns in gd");
 
 template <int N>
 struct Const {              // a compile-time number as an argument
@@ -663,8 +664,9 @@ __device__ __forceinline__ void sort_pass(const BatchDev& B, const PassScratch& 
         // lane of the current bin accumulates
         dgn.irregular += 1;
         float acc = 0.0f, nT = 0.0f, nA = 0.0f;
-        float* nc = (float*)ps.gd;               // the gas columns' new values
-        for (int c = 0; c < nE; ++c) nc[c * 32 + lane] = 0.0f;   // lanes' own entries
+        float* nc = (float*)ps.gd;               // the gas columns' new values, [column][NG]
+        if (lane < ng)
+            for (int c = 0; c < nE; ++c) nc[c * ng + lane] = 0.0f;   // lanes' own entries
         int ig = 0;
         double sum = 0.0, gp = 0.0;
 #pragma unroll 1
@@ -693,7 +695,7 @@ __device__ __forceinline__ void sort_pass(const BatchDev& B, const PassScratch& 
                 }
                 if (lane == ig)
                     for (int c = 0; c < nE; ++c)
-                        nc[c * 32 + lane] = __fadd_rn(nc[c * 32 + lane],
+                        nc[c * ng + lane] = __fadd_rn(nc[c * ng + lane],
                                                       __fmul_rn(__fmul_rn(share, ps.col[c * ng + ((q >> 5) & 31)]), w));
                 if (part == 0) {
                     sum = closes ? __dadd_rn(sum, __dmul_rn(fr, (double)w)) : __dadd_rn(sum, (double)w);
@@ -703,7 +705,7 @@ __device__ __forceinline__ void sort_pass(const BatchDev& B, const PassScratch& 
                         acc = __fdiv_rn(acc, fs);
                         nT = __fdiv_rn(nT, fs);
                         nA = __fdiv_rn(nA, fs);
-                        for (int c = 0; c < nE; ++c) nc[c * 32 + lane] = __fdiv_rn(nc[c * 32 + lane], fs);
+                        for (int c = 0; c < nE; ++c) nc[c * ng + lane] = __fdiv_rn(nc[c * ng + lane], fs);
                     }
                     if (dbg_split && lane == 0) dbg_split[ig] = (int16_t)p;
                     ig = ig + 1;
@@ -719,14 +721,14 @@ __device__ __forceinline__ void sort_pass(const BatchDev& B, const PassScratch& 
             acc = __fdiv_rn(acc, fs);
             nT = __fdiv_rn(nT, fs);
             nA = __fdiv_rn(nA, fs);
-            for (int c = 0; c < nE; ++c) nc[c * 32 + lane] = __fdiv_rn(nc[c * 32 + lane], fs);
+            for (int c = 0; c < nE; ++c) nc[c * ng + lane] = __fdiv_rn(nc[c * ng + lane], fs);
         }
         kg = acc;
         uT = nT;
         cAdd = nA;
         __syncwarp();
         if (lane < ng)
-            for (int c = 0; c < nE; ++c) ps.col[c * ng + lane] = nc[c * 32 + lane];
+            for (int c = 0; c < nE; ++c) ps.col[c * ng + lane] = nc[c * ng + lane];
         __syncwarp();
         return;
     }
