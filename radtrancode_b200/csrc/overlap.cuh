@@ -743,7 +743,7 @@ __device__ __forceinline__ void sort_pass(const BatchDev& B, const PassScratch& 
     if (nE <= 1) walk(Const<1>());
     else if (nE == 2) walk(Const<2>());
     else if (nE == 3) walk(Const<3>());
-    else walk(Const<kMaxCols - 1>());
+    else walk(Const<kMaxCols>());
     uT = cT;
     __syncwarp();
 }

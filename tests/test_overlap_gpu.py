@@ -126,3 +126,27 @@ def test_elements_across_two_boundaries(ctx, oracle, monkeypatch, ng, nabs, tile
     c64, g64, _ = oracle.cirsrtfg_wave(kt, cia, job, oracle.ORC_FP64)
     assert rad_err(c, c64) <= RAD_TOL
     assert jac_err(g, g64, job.nv) <= JAC_TOL
+
+
+@pytest.mark.parametrize("tile", [0, 8])
+@pytest.mark.parametrize("ng,nabs,nact,broad", [(5, 9, 8, False), (16, 10, 8, False), (20, 9, 8, False), (20, 9, 7, False),
+                                                (4, 9, 8, True), (6, 9, 8, True)])
+def test_eight_gas_columns(ctx, oracle, monkeypatch, ng, nabs, nact, broad, tile):
+    """Seven and eight retrieved absorbers, no temperature, and further ones
+    that are not retrieved: every column is rebinned in every pass, by the
+    walk over bins and (broad) by the sequential one."""
+    delg = np.array(_BROAD[ng], np.float32) / 32 if broad else None
+    kt, cia, job = _case_of_gases(monkeypatch, ng, nabs, delg)
+    job.xmap[:, 2 + nact:, :] = 0.0
+    ctx.set_ktables(kt)
+    ctx.set_cia(cia)
+    ctx.set_tile(tile)
+    try:
+        c, g, _ = ctx.cirsrtfg_wave(job)
+        st = ctx.stats()
+    finally:
+        ctx.set_tile(0)
+    assert (st["irregular_passes"] > 0) == broad
+    c64, g64, _ = oracle.cirsrtfg_wave(kt, cia, job, oracle.ORC_FP64)
+    assert rad_err(c, c64) <= RAD_TOL
+    assert jac_err(g, g64, job.nv) <= JAC_TOL
