@@ -223,17 +223,17 @@ __device__ __forceinline__ void interp_lin(const float* t, const KgPos& L, int g
 
 // get_kg for a wavenumber between two table points (get_kg.f:380-438):
 // 2 NG linearly interpolated values, weighted (1 - w2) delg and w2 delg,
-// rank-rebinned by rankk on lane 0.  scr: per-warp shared scratch (rankk_off).
+// rank-rebinned by rankk on lane 0.  scr: per-warp shared scratch (RankkOff).
 // Called by the whole warp.
 template <bool t2>
 __device__ void get_kg_lane_nc(const BatchDev& B, int64_t slice, float w1, float w2, const KgPos& L, int lane,
                                float* scr,
                                float& k, float& dk) {
     const int ng = B.ng;
-    const RankkOff o = rankk_off(ng);
-    float *cont = scr + o.cont, *dcont = scr + o.dcont, *fac = scr + o.fac, *tmp = scr + o.tmp;
-    float *kg = scr + o.kg, *dkg = scr + o.dkg;
-    unsigned short* ico = (unsigned short*)(scr + o.ico);
+    using Off = RankkOff;
+    float *cont = scr + Off::cont, *dcont = scr + Off::dcont, *fac = scr + Off::fac, *tmp = scr + Off::tmp;
+    float *kg = scr + Off::kg, *dkg = scr + Off::dkg;
+    unsigned short* ico = (unsigned short*)(scr + Off::ico);
     k = 0.0f;
     dk = 0.0f;
     if (slice < 0) return;

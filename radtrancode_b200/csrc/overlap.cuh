@@ -255,9 +255,14 @@ struct PassScratch {
     float2* kg;        // [gas with a table][NG]: k and dk/dT of the layer's gases
 };
 __host__ __device__ constexpr int pass_chunk(int ng) { return (ng * ng + 31) / 32; }
-// gd and rec each hold NG rows of NG + 1 words
+// gd and rec each hold NG rows of NG + 1 words, and gd the sequential walk's kMaxCols
+// rows of 32: up to NG 9 those are the most.  Rows of NG words, and rankk's arrays at
+// offsets by NG, would need no more than the elements, but the passes' instances lose
+// by it: 10-point tables, 73 layers, 3 absorbers, 515 wavenumbers take 292 us with
+// them, 276 so.
 __host__ __device__ constexpr int pass_gd_bytes(int ng) {
-    return 8 * 32 * pass_chunk(ng) > 4 * ng * (ng + 1) ? 8 * 32 * pass_chunk(ng) : (4 * ng * (ng + 1) + 15) & ~15;
+    const int pref = 8 * 32 * pass_chunk(ng), rows = (4 * ng * (ng + 1) + 15) & ~15, cols = 4 * 32 * kMaxCols;
+    return pref > rows ? (pref > cols ? pref : cols) : (rows > cols ? rows : cols);
 }
 __host__ __device__ constexpr int pass_kg_offset(int ng) { return 2 * pass_gd_bytes(ng) + 16; }
 __host__ __device__ constexpr int pass_scratch_bytes(int ng, int ncol, int ngk) {
@@ -268,14 +273,13 @@ __host__ __device__ constexpr int pass_scratch_bytes(int ng, int ncol, int ngk) 
 // derivative and weight of its 2 NG elements, 2 NG + 1 words of work, k and dk/dT of
 // the NG bins, the elements' order in 16 bits.
 struct RankkOff {
-    int cont, dcont, fac, tmp, kg, dkg, ico, bytes;
+    static constexpr int cont = 0, dcont = 2 * kMaxNg, fac = 4 * kMaxNg, tmp = 6 * kMaxNg, kg = 8 * kMaxNg + 2,
+                         dkg = kg + kMaxNg, ico = dkg + kMaxNg;
+    static constexpr int bytes(int ng) { return 4 * ico + 2 * 2 * ng; }
 };
-__host__ __device__ constexpr RankkOff rankk_off(int ng) {
-    return {0, 2 * ng, 4 * ng, 6 * ng, 8 * ng + 1, 9 * ng + 1, 10 * ng + 1, 4 * (10 * ng + 1) + 2 * 2 * ng};
-}
 constexpr bool scratch_fits() {
     for (int ng = kNgMin; ng <= kNgMax; ++ng)
-        if (rankk_off(ng).bytes > pass_scratch_bytes(ng, 0, 0) || 4 * kMaxCols * ng > pass_gd_bytes(ng)) return false;
+        if (RankkOff::bytes(ng) > pass_scratch_bytes(ng, 0, 0) || 4 * 32 * kMaxCols > pass_gd_bytes(ng)) return false;
     return true;
 }
 static_assert(scratch_fits(), "at every NG rankk's arrays lie in one warp's scratch, the sequential walk's columns in gd");
@@ -664,9 +668,8 @@ __device__ __forceinline__ void sort_pass(const BatchDev& B, const PassScratch& 
         // lane of the current bin accumulates
         dgn.irregular += 1;
         float acc = 0.0f, nT = 0.0f, nA = 0.0f;
-        float* nc = (float*)ps.gd;               // the gas columns' new values, [column][NG]
-        if (lane < ng)
-            for (int c = 0; c < nE; ++c) nc[c * ng + lane] = 0.0f;   // lanes' own entries
+        float* nc = (float*)ps.gd;               // the gas columns' new values
+        for (int c = 0; c < nE; ++c) nc[c * 32 + lane] = 0.0f;   // lanes' own entries
         int ig = 0;
         double sum = 0.0, gp = 0.0;
 #pragma unroll 1
@@ -695,7 +698,7 @@ __device__ __forceinline__ void sort_pass(const BatchDev& B, const PassScratch& 
                 }
                 if (lane == ig)
                     for (int c = 0; c < nE; ++c)
-                        nc[c * ng + lane] = __fadd_rn(nc[c * ng + lane],
+                        nc[c * 32 + lane] = __fadd_rn(nc[c * 32 + lane],
                                                       __fmul_rn(__fmul_rn(share, ps.col[c * ng + ((q >> 5) & 31)]), w));
                 if (part == 0) {
                     sum = closes ? __dadd_rn(sum, __dmul_rn(fr, (double)w)) : __dadd_rn(sum, (double)w);
@@ -705,7 +708,7 @@ __device__ __forceinline__ void sort_pass(const BatchDev& B, const PassScratch& 
                         acc = __fdiv_rn(acc, fs);
                         nT = __fdiv_rn(nT, fs);
                         nA = __fdiv_rn(nA, fs);
-                        for (int c = 0; c < nE; ++c) nc[c * ng + lane] = __fdiv_rn(nc[c * ng + lane], fs);
+                        for (int c = 0; c < nE; ++c) nc[c * 32 + lane] = __fdiv_rn(nc[c * 32 + lane], fs);
                     }
                     if (dbg_split && lane == 0) dbg_split[ig] = (int16_t)p;
                     ig = ig + 1;
@@ -721,14 +724,14 @@ __device__ __forceinline__ void sort_pass(const BatchDev& B, const PassScratch& 
             acc = __fdiv_rn(acc, fs);
             nT = __fdiv_rn(nT, fs);
             nA = __fdiv_rn(nA, fs);
-            for (int c = 0; c < nE; ++c) nc[c * ng + lane] = __fdiv_rn(nc[c * ng + lane], fs);
+            for (int c = 0; c < nE; ++c) nc[c * 32 + lane] = __fdiv_rn(nc[c * 32 + lane], fs);
         }
         kg = acc;
         uT = nT;
         cAdd = nA;
         __syncwarp();
         if (lane < ng)
-            for (int c = 0; c < nE; ++c) ps.col[c * ng + lane] = nc[c * ng + lane];
+            for (int c = 0; c < nE; ++c) ps.col[c * ng + lane] = nc[c * 32 + lane];
         __syncwarp();
         return;
     }
