@@ -19,6 +19,7 @@
 
 #include <algorithm>
 
+#include "quotient.h"
 #include "rtb_common.h"
 
 namespace rtb {
@@ -380,12 +381,12 @@ __device__ __forceinline__ void walk_bins(const PassScratch& ps, int ng, int nlo
     }
     if (!closes && lane != ng - 1) nf = 1.0f;   // the last bin reached, left open
     kg = in ? (closes || lane == ng - 1 ? __fdiv_rn(acc, nf) : acc) : 0.0f;
-    const float inv = in ? __frcp_rn(nf) : 0.0f;
-    cT = g.T * inv;
-    cAdd = g.add * inv;
+    const float inv = in && nf != 0.0f ? __frcp_rn(nf) : 0.0f;
+    cT = quotient(g.T, nf, inv);
+    cAdd = quotient(g.add, nf, inv);
 #pragma unroll
     for (int e = 0; e < NE; ++e)
-        if (e < nE && lane < ng) ps.col[e * ng + lane] = g.e[e] * inv;
+        if (e < nE && lane < ng) ps.col[e * ng + lane] = quotient(g.e[e], nf, inv);
 }
 
 // One overlap pass.  On entry lane g holds a = k1(g) [* a1], b = k2(g) * a2, the
