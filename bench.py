@@ -342,7 +342,7 @@ def batch_leg(ctx, kt, cia, nspec, nthr):
     ctx.prepare(jobs)
     t_prep = time.perf_counter() - t
     ctx.set_tile(0)
-    ctx.set_schedule(0, 0)
+    ctx.set_schedule(-1, 0)
     ctx.launch()
     ctx.fetch()
     ms_default = ctx.stats()["ms_kernel"]
@@ -357,7 +357,7 @@ def batch_leg(ctx, kt, cia, nspec, nthr):
     ms_tuned = ms[-1]
     ctx.use_graph(False)
     ctx.set_tile(0)
-    ctx.set_schedule(0, 0)
+    ctx.set_schedule(-1, 0)
     pick = np.linspace(0, nspec - 1, BATCH_ACC).astype(int)
     acc = accuracy(kt, cia, [(jobs[i], outs[i]) for i in pick], nthr, f"{BATCH_ACC} spectra of the batch")
     t = time.perf_counter()

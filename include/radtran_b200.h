@@ -401,9 +401,9 @@ int rtb_set_strict_ties(rtb_context* ctx, int on);
  *   schedule 1  dynamic: blocks pull the next item from a counter
  *   schedule 2  dynamic, items issued longest first (spectra ordered by a
  *               cost model: layers x overlap passes x gradient columns)
- * blocks_per_sm 0 = the occupancy maximum.  A context in which no schedule was
- * set chooses: 0 with fewer than two items a block, else 1, or 2 for a batch of
- * several spectra.  Results do not depend on the schedule. */
+ *   schedule -1 (the default) chosen by the batch: 0 with fewer than two items a
+ *               block, else 1, or 2 for a batch of several spectra
+ * blocks_per_sm 0 = the occupancy maximum.  Results do not depend on the schedule. */
 int rtb_fwd_set_schedule(rtb_context* ctx, int schedule, int blocks_per_sm);
 
 /* Tile shape of the resident batch's launches: warps per block, i.e. the

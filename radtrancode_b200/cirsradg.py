@@ -273,6 +273,8 @@ class Context:
         self._check(self._L.rtb_fwd_launch(self._h))
 
     def set_schedule(self, schedule, blocks_per_sm=0):
+        """Issue order of the resident batch's items (0 static, 1 counter, 2 longest first; -1 = chosen by the
+        batch) and blocks per SM (0 = the most that fit)."""
         self._check(self._L.rtb_fwd_set_schedule(self._h, schedule, blocks_per_sm))
 
     def set_tile(self, warps=0):

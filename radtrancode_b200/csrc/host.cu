@@ -1792,7 +1792,7 @@ int rtb_fwd_launch_static(rtb_context* c) { return launch_static(c); }
 
 int rtb_fwd_set_schedule(rtb_context* c, int schedule, int blocks_per_sm) {
     if (!c) return RTB_ERR_ARG;
-    if (schedule < 0 || schedule > 2 || blocks_per_sm < 0)
+    if (schedule < -1 || schedule > 2 || blocks_per_sm < 0)
         return fail(c, RTB_ERR_ARG, "schedule %d, blocks_per_sm %d", schedule, blocks_per_sm);
     c->sched = c->sched_user = schedule;
     c->occ = c->occ_user = blocks_per_sm;

@@ -27,3 +27,13 @@ def ctx():
     c = cirsradg.Context(0)
     yield c
     c.close()
+
+
+@pytest.fixture(autouse=True)
+def _form_chosen_by_the_batch(request):
+    """A test that uses the shared context leaves it with no tile and no schedule set."""
+    yield
+    if "ctx" in request.fixturenames:
+        c = request.getfixturevalue("ctx")
+        c.set_tile(0)
+        c.set_schedule(-1, 0)

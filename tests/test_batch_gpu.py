@@ -129,3 +129,27 @@ def test_autotune_of_a_small_batch_keeps_the_chosen_form(ctx):
     assert tune["candidates"] >= 10 and tune["warps"] in (2, 4, 8, 16)
     c.launch()
     _same(c.fetch(), one)
+
+
+def test_schedule_can_be_left_to_the_batch_again(ctx):
+    """set_schedule(-1, 0) after another schedule."""
+    kt, cia = synth.make_ktables([synth.CH4, synth.C2H6], np_=6, nt=5, ng=20, nbin=512, seed=3), synth.make_cia(3)
+    jobs = [synth.make_job(kt, [synth.CH4, synth.C2H6][:1 + k % 2], nlayer=n, seed=k, nwave=450)
+            for k, n in enumerate([5, 17, 9])]
+    with cirsradg.Context(0) as c:
+        c.set_ktables(kt)
+        c.set_cia(cia)
+        c.prepare(jobs)
+        c.launch()
+        chosen, grid = c.fetch(), c.stats()["grid"]
+        c.set_schedule(0, 1)
+        c.launch()
+        _same(c.fetch(), chosen)
+        assert c.stats()["grid"] < grid
+        c.set_schedule(-1, 0)
+        c.launch()
+        _same(c.fetch(), chosen)
+        assert c.stats()["grid"] == grid
+        for schedule in (-2, 3):
+            with pytest.raises(cirsradg.RtbError, match="ARG"):
+                c.set_schedule(schedule, 0)
