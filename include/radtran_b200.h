@@ -408,9 +408,9 @@ int rtb_fwd_set_schedule(rtb_context* ctx, int schedule, int blocks_per_sm);
 
 /* Tile shape of the resident batch's launches: warps per block, i.e. the
  * layers of one (spectrum, wavenumber) item worked on at once (one warp per
- * layer, one lane per g-ordinate): 2, 4 or 8; 0 (the default) = chosen by the
+ * layer, one lane per g-ordinate): 2, 4, 8 or 16; 0 (the default) = chosen by the
  * batch: 8, or 16 where there are no more items than SMs, several blocks sharing
- * an item where more SMs would be idle.  Tiles 2 and 4 exist for the usual kernel
+ * an item where more SMs would be idle (with a tile set, none do).  Tiles 2 and 4 exist for the usual kernel
  * instance (one temperature grid, no para-H2 / IMOD 18 / iform / non-LTE /
  * air-Rayleigh option); other batches run 8.  Results do not depend on the tile. */
 int rtb_fwd_set_tile(rtb_context* ctx, int warps);

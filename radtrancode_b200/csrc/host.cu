@@ -1803,8 +1803,8 @@ int rtb_fwd_set_schedule(rtb_context* c, int schedule, int blocks_per_sm) {
 
 int rtb_fwd_set_tile(rtb_context* c, int warps) {
     if (!c) return RTB_ERR_ARG;
-    if (!(warps == 0 || warps == 2 || warps == 4 || warps == 8))
-        return fail(c, RTB_ERR_ARG, "tile of %d warps per block (2, 4 or 8)", warps);
+    if (!(warps == 0 || warps == 2 || warps == 4 || warps == 8 || warps == kTileWide))
+        return fail(c, RTB_ERR_ARG, "tile of %d warps per block (2, 4, 8 or 16)", warps);
     c->tile = c->tile_user = warps;
     if (!c->prepared) return RTB_OK;
     CUDA_TRY(c, cudaSetDevice(c->device));

@@ -131,8 +131,9 @@ def test_autotune_of_a_small_batch_keeps_the_chosen_form(ctx):
     _same(c.fetch(), one)
 
 
-def test_schedule_can_be_left_to_the_batch_again(ctx):
-    """set_schedule(-1, 0) after another schedule."""
+def test_schedule_and_tile_can_be_left_to_the_batch_again(ctx):
+    """set_schedule(-1, 0) after another schedule, and every tile that the
+    autotuner reports set by hand, 16 warps with several items a block included."""
     kt, cia = synth.make_ktables([synth.CH4, synth.C2H6], np_=6, nt=5, ng=20, nbin=512, seed=3), synth.make_cia(3)
     jobs = [synth.make_job(kt, [synth.CH4, synth.C2H6][:1 + k % 2], nlayer=n, seed=k, nwave=450)
             for k, n in enumerate([5, 17, 9])]
@@ -150,6 +151,12 @@ def test_schedule_can_be_left_to_the_batch_again(ctx):
         c.launch()
         _same(c.fetch(), chosen)
         assert c.stats()["grid"] == grid
+        for tile in (2, 4, 8, 16):
+            c.set_tile(tile)
+            c.launch()
+            _same(c.fetch(), chosen)
         for schedule in (-2, 3):
             with pytest.raises(cirsradg.RtbError, match="ARG"):
                 c.set_schedule(schedule, 0)
+        with pytest.raises(cirsradg.RtbError, match="ARG"):
+            c.set_tile(32)
