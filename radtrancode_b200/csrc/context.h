@@ -179,6 +179,7 @@ struct rtb_context {
     int debug = 0;
     cudaStream_t user_stream = nullptr;   // caller-provided stream (NULL: own stream)
     // resident batch (rtb_fwd_prepare)
+    int static_loaded = 0;                // the static scratch is on the device (prepare_ex)
     int prepared = 0;
     int placed = 0;                       // outputs of the resident batch go to caller device arrays
     rtb::BatchDev B{};

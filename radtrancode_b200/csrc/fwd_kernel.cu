@@ -30,13 +30,17 @@
 #include "overlap.cuh"
 #include "rtb_common.h"
 
+#ifndef FWD_PART
+#error "FWD_PART: 0, the host side, or 1 to 13, a part of the instances"
+#endif
+
 namespace rtb {
 
 namespace {
 
 // NR heapsort of radtran/cirsradg/sort2g.f:1-52 on shared memory (one thread);
 // ra/ib hold RA(1..n)/IB(1..n) at ra[0..n-1].
-__device__ __noinline__ void heapsort_sort2g(int n, float* ra0, unsigned short* ib0) {
+static __device__ __noinline__ void heapsort_sort2g(int n, float* ra0, unsigned short* ib0) {
     if (n < 2) return;
     float* RA = ra0 - 1;
     unsigned short* IB = ib0 - 1;
@@ -121,7 +125,7 @@ __host__ __device__ inline Layout make_layout(int ng, int nsw, int ncol, int ngk
 // ordinates and distribution summed in the reference's order, the `<=` test,
 // the split fraction and the ig <= ng guards.  cont/dcont/weight are sorted
 // and permuted in place (sort2g heapsort); ico is scratch.
-__device__ void rankk_lane(int ng, const float* gw, int nloop, float* cont, float* dcont, float* weight,
+static __device__ void rankk_lane(int ng, const float* gw, int nloop, float* cont, float* dcont, float* weight,
                                         unsigned short* ico, float* tmp, float* k_g, float* dkdt) {
     float g_ord[kMaxNg + 1];
     g_ord[0] = 0.0f;
@@ -314,7 +318,7 @@ __device__ __forceinline__ void e3interp_dev(const double* tab, double x, double
 // the wavenumber index in cirsradg_wave.f:933-935, never 0, so planck_wave
 // and invplanck_wave take their wavelength branch (y = 1e4 / v) there.
 // DOUBLE inside as those two are; REAL factors as calc_nlte_t forms them.
-__device__ __noinline__ float nlte_temp(int inlte, float T, float p, float v, float k1, float A) {
+static __device__ __noinline__ float nlte_temp(int inlte, float T, float p, float v, float k1, float A) {
     float f;
     if (inlte == 1) {
         const float ntot = __fmul_rn(__fdiv_rn(__fmul_rn(p, 101325.0f), __fmul_rn(1.380658e-23f, T)), 1.0e-6f);
@@ -340,7 +344,7 @@ __device__ __noinline__ float nlte_temp(int inlte, float T, float p, float v, fl
 // iform = 3 on an IMOD 3 path (cirsradg_wave.f:913-929): the total flux of the
 // planet, every term of lane g's radiance and derivatives times x.  Out of
 // line, as is path_imod18: the common paths' code stays as compact as it was.
-__device__ __noinline__ void scale_path(float x, int nlays, int ng, int g, float* drdt, float* trd, float* rad,
+static __device__ __noinline__ void scale_path(float x, int nlays, int ng, int g, float* drdt, float* trd, float* rad,
                                         float* gts) {
     rad[g] *= x;
     gts[g] *= x;
@@ -357,7 +361,7 @@ __device__ __noinline__ void scale_path(float x, int nlays, int ng, int g, float
 // dR/dtau_j = c (B_j G_j + sum_{m>j} B_m (G_m - G_{m-1})), G_m = E3'(T_m) T_m
 // (the reference leaves the surface term out of the derivative).  drdt
 // receives dR/dtau_j, trd the factor of dB/dT in the temperature column.
-__device__ __noinline__ void path_imod18(const double* e3tab, float xfac18, int nlays, int ng, int g,
+static __device__ __noinline__ void path_imod18(const double* e3tab, float xfac18, int nlays, int ng, int g,
                                          const int* layinc, const float* scale, const float* tau_s,
                                          const float* bb, float radground_s, float gradground_s, float* drdt,
                                          float* trd, float* rad, float* gts) {
@@ -410,7 +414,7 @@ __device__ __forceinline__ void cia_bilinear(const float* kc, int64_t e, int64_t
 
 // RAYLEIGHA (radtran/scatter/rayleigha.f:1-38): the Rayleigh cross section of
 // air at pressure P (atm) and temperature T, REAL arithmetic in its order
-__device__ __noinline__ float rayleigha_dev(float v, float P, float T) {
+static __device__ __noinline__ float rayleigha_dev(float v, float P, float T) {
     const float c1 = 8342.12f, c2 = 2406030.0f, c3 = 15997.0f, delta = 0.035f, pi = 3.1415927f, k = 1.37971e-23f;
     float lambda = __fdiv_rn(1e4f, v);
     const float nu2 = __fdiv_rn(1.0f, __fmul_rn(lambda, lambda));
@@ -1040,21 +1044,21 @@ fwd_kernel(BatchDev B, int nsw_max, int ncol_max, int ngk_max, int nlmax_max, in
     if (tid < 5 && s_count[tid]) atomicAdd(B.counters + tid, s_count[tid]);
 }
 
-// host-side helpers exported to host.cu
-size_t fwd_merge_table_bytes() { return sizeof(MergeLane) * kMergeLevels * 32; }
-void fwd_merge_table(int ng, void* table) {
-    for (int i = 0; i < kMergeLevels * 32; ++i) ((MergeLane*)table)[i] = merge_lane(ng, i / 32, i % 32);
-}
-
-int fwd_smem_bytes(int ng, int nsw, int ncol, int ngk, int nlmax, int npath, int warps) {
-    return make_layout(ng, nsw, ncol, ngk, nlmax, npath, warps).total;
-}
-
-namespace {
+// The instances are compiled in parts, this file with FWD_PART = 1 .. 13: each part
+// is a module of its own, which CUDA loads at the first use of one of its kernels.
+// In one module of all 47 a process's first call took 37 ms, 31 of them for loading
+// it.  The host side is FWD_PART = 0.  Parts 1-4, 5-8 and 9-12: 8 warps, 16 warps and
+// pairs, by t2 + 2 ext; part 13: 2 and 4 warps.
 using FwdKern = void (*)(BatchDev, int, int, int, int, int);
-// the instance of a launch: t2 and ext as the batch needs them; tiles of 2 and 4
-// warps, and NG = 20 as a constant, exist for the usual instance only (one
-// temperature grid, no extended options).  Up to 256 elements a pass are
+#define RTB_FWD_PARTS(X) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13)
+#define RTB_FWD_PART_DECL(p) FwdKern fwd_part_##p(int warps, int ng);
+RTB_FWD_PARTS(RTB_FWD_PART_DECL)
+
+#if FWD_PART > 0
+namespace {
+// the instance of a part for an NG: tiles of 2 and 4 warps, and NG = 20 as a
+// constant, exist for the usual options only (one temperature grid, no extended
+// options).  Up to 256 elements a pass are
 // sorted in registers, more are merged in shared memory: one spectrum of
 // 16-point tables (80 layers, 150 wavenumbers, 2 absorbers, a block an item) takes
 // 0.22 ms by the first and 0.27 ms by the second, one of 20-point tables (120
@@ -1067,17 +1071,41 @@ FwdKern fwd_by_ng(int ng) {
     if (ng * ng > 128) return fwd_kernel<t2, ext, WARPS, -8, CL>;
     return fwd_kernel<t2, ext, WARPS, -4, CL>;
 }
-template <int WARPS, int CL = 1>
-FwdKern fwd_by_options(bool t2, bool ext, int ng) {
-    if (ext) return t2 ? fwd_by_ng<true, true, WARPS, CL>(ng) : fwd_by_ng<false, true, WARPS, CL>(ng);
-    return t2 ? fwd_by_ng<true, false, WARPS, CL>(ng) : fwd_by_ng<false, false, WARPS, CL>(ng);
+template <int part>
+FwdKern fwd_of_part(int warps, int ng) {
+    constexpr bool t2 = (part - 1) & 1, ext = (part - 1) & 2;
+    if constexpr (part <= 4) return fwd_by_ng<t2, ext, kTileDefault>(ng);
+    if constexpr (part > 4 && part <= 8) return fwd_by_ng<t2, ext, kTileWide>(ng);
+    if constexpr (part > 8 && part <= 12) return fwd_by_ng<t2, ext, kTileDefault, 2>(ng);
+    if constexpr (part == 13) return warps == 2 ? fwd_by_ng<false, false, 2>(ng) : fwd_by_ng<false, false, 4>(ng);
 }
+}  // namespace
+#define RTB_FWD_PART_NAME2(p) fwd_part_##p
+#define RTB_FWD_PART_NAME(p) RTB_FWD_PART_NAME2(p)
+FwdKern RTB_FWD_PART_NAME(FWD_PART)(int warps, int ng) { return fwd_of_part<FWD_PART>(warps, ng); }
+
+#else
+// host-side helpers exported to host.cu
+size_t fwd_merge_table_bytes() { return sizeof(MergeLane) * kMergeLevels * 32; }
+void fwd_merge_table(int ng, void* table) {
+    for (int i = 0; i < kMergeLevels * 32; ++i) ((MergeLane*)table)[i] = merge_lane(ng, i / 32, i % 32);
+}
+
+int fwd_smem_bytes(int ng, int nsw, int ncol, int ngk, int nlmax, int npath, int warps) {
+    return make_layout(ng, nsw, ncol, ngk, nlmax, npath, warps).total;
+}
+
+namespace {
+// the instance of a launch: t2 and ext as the batch needs them
 FwdKern fwd_instance(bool t2, bool ext, int warps, int ng, bool pair) {
-    if (warps == kTileWide) return fwd_by_options<kTileWide>(t2, ext, ng);
-    if (pair) return fwd_by_options<kTileDefault, 2>(t2, ext, ng);
-    if (warps == 2 && !t2 && !ext) return fwd_by_ng<false, false, 2>(ng);
-    if (warps == 4 && !t2 && !ext) return fwd_by_ng<false, false, 4>(ng);
-    return fwd_by_options<kTileDefault>(t2, ext, ng);
+    static constexpr FwdKern (*parts[])(int, int) = {
+#define RTB_FWD_PART_PTR(p) fwd_part_##p,
+        RTB_FWD_PARTS(RTB_FWD_PART_PTR)};
+    const int options = (t2 ? 1 : 0) + (ext ? 2 : 0);
+    if (warps == kTileWide) return parts[4 + options](warps, ng);
+    if (pair) return parts[8 + options](warps, ng);
+    if ((warps == 2 || warps == 4) && !options) return parts[12](warps, ng);
+    return parts[options](warps, ng);
 }
 }  // namespace
 
@@ -1142,5 +1170,7 @@ cudaError_t launch_fwd(const BatchDev& B, int nsw, int ncol, int ngk, int nlmax,
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kern, B, nsw, ncol, ngk, nlmax, npath);
 }
+
+#endif  // FWD_PART
 
 }  // namespace rtb

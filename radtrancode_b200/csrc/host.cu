@@ -1005,6 +1005,12 @@ static void longest_first(const rtb_context* c, std::vector<int>& order) {
         for (int64_t it = c->item_start_host[s]; it < c->item_start_host[s + 1]; ++it) order.push_back((int)it);
 }
 
+// Scratch of rtb_fwd_launch_static: one fixed array per device, part of the
+// library's device image, so that the call never goes to the allocator.  The
+// kernel writes every entry of a slot before it reads it, so nothing here has
+// to start at zero.
+static __device__ __align__(256) float g_fwd_static_scratch[RTB_STATIC_SCRATCH_BYTES / sizeof(float)];
+
 // pack + upload a batch; the device copy stays resident until the next prepare
 int prepare_ex(rtb_context* c, int nspec, const rtb_atm* atms, const OutPlace* place) {
     if (!c || nspec <= 0 || !atms) return fail(c, RTB_ERR_ARG, "bad batch arguments");
@@ -1013,6 +1019,12 @@ int prepare_ex(rtb_context* c, int nspec, const rtb_atm* atms, const OutPlace* p
         return fail(c, RTB_ERR_UNSUPPORTED, "NG=%d outside the device range %d..%d", c->ng, kNgMin, kNgMax);
     CUDA_TRY(c, cudaSetDevice(c->device));
     c->prepared = 0;
+    if (!c->static_loaded) {
+        // the module of the static scratch takes its device memory now, not at the first launch into it
+        void* p = nullptr;
+        if (cudaGetSymbolAddress(&p, g_fwd_static_scratch) != cudaSuccess) cudaGetLastError();
+        c->static_loaded = 1;
+    }
     // instrument convolution of each spectrum's outputs (cirsrtfg_wave.f:448-516)
     std::vector<ConvSpec> convs(nspec);
     int any_conv = 0;
@@ -1452,12 +1464,6 @@ int run_batch(rtb_context* c, int nspec, const rtb_atm* atms, float* const* calc
     if (r) return r;
     return fetch(c, calcout, gradients, gradtsurf);
 }
-
-// Scratch of rtb_fwd_launch_static: one fixed array per device, part of the
-// library's device image, so that the call never goes to the allocator.  The
-// kernel writes every entry of a slot before it reads it, so nothing here has
-// to start at zero.
-static __device__ __align__(256) float g_fwd_static_scratch[RTB_STATIC_SCRATCH_BYTES / sizeof(float)];
 
 constexpr int kMaxStaticDevices = 64;
 std::mutex g_static_mu;

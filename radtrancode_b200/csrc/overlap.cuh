@@ -44,7 +44,7 @@ __device__ __forceinline__ float wkey(unsigned long long w) { return __uint_as_f
 // exactly its order.  The sift-down loads the four grandchildren while it
 // compares the two children, so that no shared-memory load is on the critical
 // path of a level.
-__device__ __noinline__ void heapsort_words(int n, unsigned long long* W0) {
+static __device__ __noinline__ void heapsort_words(int n, unsigned long long* W0) {
     if (n < 2) return;
     unsigned long long* W = W0 - 1;            // W[1..n]
     int L = n / 2 + 1, IR = n;
