@@ -22,7 +22,7 @@ int fwd_tile_warps(bool t2, bool ext, int warps);
 // the overlap merge's per-level, per-lane table of an NG (MergeLane)
 size_t fwd_merge_table_bytes();
 void fwd_merge_table(int ng, void* table);
-int fwd_blocks_per_sm(int smem, bool t2, bool ext, int warps, int ng);
+int fwd_blocks_per_sm(int smem, bool t2, bool ext, int warps, int ng, bool pair);
 int fwd_max_clusters(int smem, bool t2, bool ext, int warps, int ng, int size);   // resident at once
 cudaError_t launch_fwd(const BatchDev& B, int nsw, int ncol, int ngk, int nlmax, int npath, int grid, int warps,
                        cudaStream_t st);
@@ -143,6 +143,7 @@ int conv_run(rtb_context* c, const ConvSpec& cs, int nseg, const ConvSeg* seg, c
 struct rtb_context {
     int device = 0;
     int nsm = 0;
+    int smem_block = 0, smem_sm = 0, smem_reserved = 0;   // shared memory of a block and of an SM, the share of each block taken by the system
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     std::string err;
@@ -197,8 +198,8 @@ struct rtb_context {
     rtb::DevBuf d_conv, d_convout;
     rtb::DevBuf d_layer;                  // rtb_layerg inputs, arguments and outputs
     std::vector<char> h_conv;
-    // fwd_blocks_per_sm by (shared bytes, t2, ext, tile, NG), a query of the driver per tile and call otherwise;
-    // fwd_max_clusters with tile x (1 + cluster size)
+    // tile_blocks by (shared bytes, t2, ext, tile, NG), pairs with 64 + tile, and max_clusters with 128 + size: else
+    // queries of the driver on every call
     std::map<std::array<int, 5>, int> bpsm_known;
     size_t dbg_perm_n = 0, dbg_split_n = 0;
     rtb_fwd_stats stats{};
@@ -211,7 +212,6 @@ struct rtb_context {
     // the caller's own choices (rtb_fwd_set_tile / rtb_fwd_set_schedule), which a batch of an untuned shape uses
     int tile_user = 0, sched_user = -1, occ_user = 0;
     int tile_eff = rtb::kTileDefault;           // warps per CTA of the resident batch's launches
-    int bpsm_w[rtb::kTileWide + 1] = {};  // blocks per SM of the batch at 2, 4, 8, 16 warps per CTA (0: not resident)
     int bpsm_max = 1;                     // blocks per SM of the current tile
     // rtb_fwd_autotune results by batch shape (layer bucket of 20, gas count): tile, schedule, occupancy
     std::map<std::pair<int, int>, std::array<int, 3>> tuned;

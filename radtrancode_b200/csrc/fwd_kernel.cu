@@ -1114,9 +1114,9 @@ int fwd_tile_warps(bool t2, bool ext, int warps) {
     return (ext || t2 || (warps != 2 && warps != 4)) ? kTileDefault : warps;
 }
 
-int fwd_blocks_per_sm(int smem, bool t2, bool ext, int warps, int ng) {
+int fwd_blocks_per_sm(int smem, bool t2, bool ext, int warps, int ng, bool pair) {
     const int w = fwd_tile_warps(t2, ext, warps);
-    const FwdKern k = fwd_instance(t2, ext, w, ng, false);
+    const FwdKern k = fwd_instance(t2, ext, w, ng, pair);
     int n = 0;
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, w * 32, smem) != cudaSuccess)

@@ -1011,6 +1011,45 @@ static void longest_first(const rtb_context* c, std::vector<int>& order) {
 // to start at zero.
 static __device__ __align__(256) float g_fwd_static_scratch[RTB_STATIC_SCRATCH_BYTES / sizeof(float)];
 
+// shared memory of a block of the resident batch's launches
+int tile_smem(const rtb_context* c, int w) {
+    return fwd_smem_bytes(c->ng, c->nsw_max, c->ncol_max, c->ngk_max, c->nlmax_max, c->npath_max, w);
+}
+
+// blocks of w warps an SM holds at most, by its 24 warps (fwd_kernel's launch
+// bounds; one block of the wide tile) and its shared memory; 0: not for this batch
+int tile_bound(const rtb_context* c, int w) {
+    const int smem = tile_smem(c, w);
+    if (smem > c->smem_block || fwd_tile_warps(c->B.t2, c->B.ext, w) != w) return 0;
+    return std::min(w == kTileWide ? 1 : 24 / w, c->smem_sm / (smem + c->smem_reserved));
+}
+
+// blocks per SM of the resident batch's launches with a tile (pair: of its
+// instance for two blocks an item).  Asking loads the instance, so it is asked
+// where one is chosen: a launch loads nothing, one that never runs is not loaded.
+int tile_blocks(rtb_context* c, int w, bool pair = false) {
+    const int bound = tile_bound(c, w);
+    if (bound <= 0) return 0;
+    const int smem = tile_smem(c, w);
+    const std::array<int, 5> key = {smem, c->B.t2, c->B.ext, pair ? 64 + w : w, c->ng};
+    const auto known = c->bpsm_known.find(key);
+    if (known != c->bpsm_known.end()) return known->second;
+    const int n = std::min(bound, fwd_blocks_per_sm(smem, c->B.t2, c->B.ext, w, c->ng, pair));
+    if (c->bpsm_known.size() < 256) c->bpsm_known[key] = n;
+    return n;
+}
+
+// clusters of `size` blocks of the wide tile that the device runs at once
+int max_clusters(rtb_context* c, int size) {
+    const int smem = tile_smem(c, kTileWide);
+    const std::array<int, 5> key = {smem, c->B.t2, c->B.ext, 128 + size, c->ng};
+    const auto known = c->bpsm_known.find(key);
+    if (known != c->bpsm_known.end()) return known->second;
+    const int n = fwd_max_clusters(smem, c->B.t2, c->B.ext, kTileWide, c->ng, size);
+    if (c->bpsm_known.size() < 256) c->bpsm_known[key] = n;
+    return n;
+}
+
 // pack + upload a batch; the device copy stays resident until the next prepare
 int prepare_ex(rtb_context* c, int nspec, const rtb_atm* atms, const OutPlace* place) {
     if (!c || nspec <= 0 || !atms) return fail(c, RTB_ERR_ARG, "bad batch arguments");
@@ -1038,30 +1077,9 @@ int prepare_ex(rtb_context* c, int nspec, const rtb_atm* atms, const OutPlace* p
     Staging st;
     const int r0 = pack_batch(c, nspec, atms, st);
     if (r0) return r0;
-    int smem_max = 0;
-    CUDA_TRY(c, cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
-    const bool t2 = c->nt < 0, ext = st.any_para || st.any_ext;
-    int bpsm_all = 0;
-    for (int w : {2, 4, 8, kTileWide}) {
-        const int sm_w = fwd_smem_bytes(c->ng, st.nsw_max, st.ncol_max, st.ngk_max, st.nlmax_max, st.npath_max, w);
-        if (sm_w > smem_max || fwd_tile_warps(t2, ext, w) != w) {
-            c->bpsm_w[w] = 0;
-        } else {
-            const std::array<int, 5> key = {sm_w, t2, ext, w, c->ng};
-            const auto known = c->bpsm_known.find(key);
-            if (known != c->bpsm_known.end()) {
-                c->bpsm_w[w] = known->second;
-            } else {
-                c->bpsm_w[w] = fwd_blocks_per_sm(sm_w, t2, ext, w, c->ng);
-                if (c->bpsm_known.size() < 256) c->bpsm_known[key] = c->bpsm_w[w];
-            }
-        }
-        bpsm_all = std::max(bpsm_all, c->bpsm_w[w]);
-    }
     const int smem = fwd_smem_bytes(c->ng, st.nsw_max, st.ncol_max, st.ngk_max, st.nlmax_max, st.npath_max, kTileDefault);
-    if (smem > smem_max)
-        return fail(c, RTB_ERR_UNSUPPORTED, "spectrum needs %d B of shared memory (device %d)", smem, smem_max);
-    if (c->bpsm_w[kTileDefault] <= 0) return fail(c, RTB_ERR_CUDA, "forward kernel cannot be resident (smem %d B)", smem);
+    if (smem > c->smem_block)
+        return fail(c, RTB_ERR_UNSUPPORTED, "spectrum needs %d B of shared memory (device %d)", smem, c->smem_block);
     // first device spectrum of each caller spectrum (path groups follow it)
     std::vector<int> first(nspec + 1, 0);
     for (int sp = 0; sp < nspec; ++sp) first[sp + 1] = first[sp] + st.nsub[sp];
@@ -1206,26 +1224,24 @@ int prepare_ex(rtb_context* c, int nspec, const rtb_atm* atms, const OutPlace* p
         B.dbg_perm = (int16_t*)c->d_dbg_perm.p;
         B.dbg_split = (int16_t*)c->d_dbg_split.p;
     }
-    // the scratch holds a slot for every block of the largest grid any tile launches
-    int64_t grid = (int64_t)c->nsm * bpsm_all;
-    if (grid > B.nitems) grid = B.nitems;
-    c->grid = (int)grid;
-    c->tile_eff = kTileDefault;
-    c->bpsm_max = c->bpsm_w[kTileDefault];
     // one scratch slot per CTA: tau[Lmax][ng] + dtau[Lmax][nsw][ng]
     B.cell_Lmax = st.Lmax;
     B.cell_slot = (int64_t)st.Lmax * c->ng * (1 + st.nsw_max);
     B.nc_off = B.cell_slot;
     if (st.any_noncoinc) B.cell_slot += (int64_t)st.Lmax * st.ngas_max * kMaxNg * 2;
     B.cell_slot = (B.cell_slot + 63) & ~(int64_t)63;
-    CUDA_TRY(c, c->d_cells.ensure((size_t)grid * B.cell_slot * sizeof(float)));
-    B.cell_scratch = (float*)c->d_cells.p;
     c->Lmax = st.Lmax;
     c->nsw_max = st.nsw_max;
     c->ncol_max = st.ncol_max;
     c->ngk_max = st.ngk_max;
     c->nlmax_max = st.nlmax_max;
     c->npath_max = st.npath_max;
+    // the scratch holds a slot for every block of the largest grid any tile launches
+    int blocks = 1;
+    for (int w : {2, 4, kTileDefault, kTileWide}) blocks = std::max(blocks, tile_bound(c, w));
+    const size_t slots = (size_t)std::min<int64_t>((int64_t)c->nsm * blocks, std::max<int64_t>(B.nitems, 1));
+    CUDA_TRY(c, c->d_cells.ensure(slots * B.cell_slot * sizeof(float)));
+    B.cell_scratch = (float*)c->d_cells.p;
     c->spec_host.clear();
     for (int s = 0; s < nspec; ++s) c->spec_host.push_back(st.spec[first[s]]);   // outputs start at path 0
     c->spec_conv = std::move(convs);
@@ -1262,7 +1278,9 @@ int prepare_ex(rtb_context* c, int nspec, const rtb_atm* atms, const OutPlace* p
         c->sched = c->sched_user;
         c->occ = c->occ_user;
     }
-    return apply_schedule(c);
+    const int r = apply_schedule(c);
+    if (r) c->prepared = 0;
+    return r;
 }
 
 void drop_graph(rtb_context* c) {
@@ -1270,18 +1288,6 @@ void drop_graph(rtb_context* c) {
     if (c->graph) cudaGraphDestroy(c->graph);
     c->gexec = nullptr;
     c->graph = nullptr;
-}
-
-// clusters of `size` blocks of the wide tile that the device runs at once
-int max_clusters(rtb_context* c, int size) {
-    const bool t2 = c->B.t2, ext = c->B.ext;
-    const int smem = fwd_smem_bytes(c->ng, c->nsw_max, c->ncol_max, c->ngk_max, c->nlmax_max, c->npath_max, kTileWide);
-    const std::array<int, 5> key = {smem, t2, ext, kTileWide * (1 + size), c->ng};
-    const auto known = c->bpsm_known.find(key);
-    if (known != c->bpsm_known.end()) return known->second;
-    const int n = fwd_max_clusters(smem, t2, ext, kTileWide, c->ng, size);
-    if (c->bpsm_known.size() < 256) c->bpsm_known[key] = n;
-    return n;
 }
 
 // grid, work counter and issue order of the resident batch from (sched, occ)
@@ -1299,8 +1305,18 @@ int apply_schedule(rtb_context* c) {
     // absorbers, 222 wavenumbers 592 and 545 us.
     const bool wide = !c->tile && B.nitems <= c->nsm;
     const int w = fwd_tile_warps(B.t2, B.ext, c->tile ? c->tile : (wide ? kTileWide : kTileDefault));
-    c->tile_eff = c->bpsm_w[w] > 0 ? w : kTileDefault;
-    c->bpsm_max = c->bpsm_w[c->tile_eff];
+    // pairs, which fit as single blocks do, first: where they run nothing else is loaded
+    const bool pair = !c->tile && !wide && c->sched < 1 && c->occ <= 0 &&
+                      2 * (int64_t)B.nitems <= (int64_t)c->nsm * tile_bound(c, kTileDefault) &&
+                      2 * (int64_t)B.nitems <= (int64_t)c->nsm * tile_blocks(c, kTileDefault, true);
+    c->tile_eff = w;
+    c->bpsm_max = tile_blocks(c, w, pair);
+    if (c->bpsm_max <= 0) {
+        c->tile_eff = kTileDefault;
+        c->bpsm_max = tile_blocks(c, kTileDefault);
+    }
+    if (c->bpsm_max <= 0)
+        return fail(c, RTB_ERR_CUDA, "forward kernel cannot be resident (smem %d B)", tile_smem(c, kTileDefault));
     const int b = c->occ > 0 ? std::min(c->occ, c->bpsm_max) : c->bpsm_max;
     int64_t grid = (int64_t)c->nsm * b;
     if (grid > B.nitems) grid = B.nitems;
@@ -1310,8 +1326,7 @@ int apply_schedule(rtb_context* c) {
         while (B.cluster < 8 && 2 * B.cluster * B.nitems <= c->nsm && B.cluster < c->Lmax &&
                B.nitems <= max_clusters(c, 2 * B.cluster))
             B.cluster *= 2;
-    if (!c->tile && !wide && c->sched < 1 && c->occ <= 0 && 2 * (int64_t)B.nitems <= (int64_t)c->nsm * b)
-        B.cluster = 2;
+    if (pair) B.cluster = 2;
     // no schedule asked for: from two items a block on they are pulled from the
     // counter, the longest spectra of several first; below that the counter's
     // round trip costs more than it evens out.  14 spectra, 7000 items of 444
@@ -1528,6 +1543,9 @@ int rtb_create(int device, rtb_context** out) {
     c->device = device;
     if (cudaSetDevice(device) != cudaSuccess) { delete c; return RTB_ERR_CUDA; }
     cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, device);
+    cudaDeviceGetAttribute(&c->smem_block, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    cudaDeviceGetAttribute(&c->smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device);
+    cudaDeviceGetAttribute(&c->smem_reserved, cudaDevAttrReservedSharedMemoryPerBlock, device);
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess) {
         delete c;
@@ -1824,7 +1842,7 @@ int rtb_fwd_autotune(rtb_context* c, rtb_fwd_tune* out) {
     const int keep_graph = c->use_graph;
     c->use_graph = 0;
     float best = 3.4e38f;
-    int best_w = kTileDefault, best_s = 0, best_b = c->bpsm_w[kTileDefault], n = 0;
+    int best_w = kTileDefault, best_s = 0, best_b = 0, n = 0;
     auto time_it = [&](int w, int sch, int b) {
         c->tile = w;
         c->sched = sch;
@@ -1848,8 +1866,8 @@ int rtb_fwd_autotune(rtb_context* c, rtb_fwd_tune* out) {
         return (int)RTB_OK;
     };
     for (int w : {4, 8, 2}) {
-        if (fwd_tile_warps(c->B.t2, c->B.ext, w) != w || c->bpsm_w[w] <= 0) continue;
-        const int bmax = c->bpsm_w[w];
+        const int bmax = tile_blocks(c, w);
+        if (bmax <= 0) continue;
         for (int sch = 0; sch <= 2; ++sch)
             for (int b = bmax; b >= 1 && b >= bmax - 2; --b)
                 if (const int r = time_it(w, sch, b)) return r;

@@ -160,3 +160,23 @@ def test_schedule_and_tile_can_be_left_to_the_batch_again(ctx):
                 c.set_schedule(schedule, 0)
         with pytest.raises(cirsradg.RtbError, match="ARG"):
             c.set_tile(32)
+
+
+# a cluster of 8 and of 2 blocks of 16 warps, one of 16, a pair of 8, one of 8: in a fresh context, whose first launch of the form is captured
+@pytest.mark.parametrize("nwave", [1, 60, 100, 150, 230])
+def test_first_launch_of_a_form_captured(ctx, nwave):
+    kt, cia = synth.make_ktables([synth.CH4, synth.C2H6], np_=6, nt=5, ng=12, nbin=256, seed=12), synth.make_cia(12)
+    job = synth.make_job(kt, [synth.CH4, synth.C2H6], nlayer=23, seed=nwave, nwave=nwave)
+    ctx.set_ktables(kt)
+    ctx.set_cia(cia)
+    ctx.set_tile(8)
+    ctx.set_schedule(0, 0)
+    one = [ctx.cirsrtfg_wave(job)]
+    with cirsradg.Context(0) as c:
+        c.set_ktables(kt)
+        c.set_cia(cia)
+        c.use_graph(True)
+        c.prepare([job])
+        for _ in range(2):                   # capture, then a replay
+            c.launch()
+            _same(c.fetch(), one)
