@@ -152,7 +152,7 @@ int rtb_calc_gain_matrix(rtb_context* c, int nx, int ny, int ldx, int ldy, const
     CUDA_TRY(c, cudaMemcpyAsync(se, sei, (size_t)ny * 8, cudaMemcpyHostToDevice, st));
     // C(a, b) = sum_i K(i, a) Se^-1(i) K(i, b) + Sa^-1(a, b)   (Sa^-1 stored column-major = (b, a) row-major)
     CUDA_TRY(c, (gemm<float, float>(nx, nx, ny, kt, ny, 1, kt, 1, ny, se, nullptr, sai, 1, nx, C, nx, 1, st)));
-    CUDA_TRY(c, launch_spd_inverse(C, Ci, nx, 0, 1, status, st));
+    CUDA_TRY(c, launch_spd_inverse(C, Ci, nx, 0, 1, c->nsm, status, st));
     // D(a, i) = Se^-1(i) sum_b C^-1(a, b) K(i, b)
     CUDA_TRY(c, (gemm<double, float>(nx, ny, nx, Ci, nx, 1, kt, ny, 1, nullptr, se, nullptr, 0, 0, D, 1, nx, st)));
     // AA(a, b) = sum_i D(a, i) K(i, b)

@@ -757,12 +757,12 @@ cudaError_t launch_phi(const PhiDev* d_ret, int nret, float* d_phi, float* d_chi
     return cudaGetLastError();
 }
 
-cudaError_t launch_spd_inverse(const double* d_a, double* d_ainv, int n, int64_t stride, int nret,
+cudaError_t launch_spd_inverse(const double* d_a, double* d_ainv, int n, int64_t stride, int nret, int nsm,
                                unsigned* d_status, cudaStream_t st) {
     if (nret <= 0) return cudaSuccess;
     const int smem = n * c_ld(n) * 8 + kNp * 8;
     // blocks per matrix: one column per warp while the batch leaves SMs idle
-    const int split = std::max(1, std::min((n + kNw - 1) / kNw, 148 / nret));
+    const int split = std::max(1, std::min((n + kNw - 1) / kNw, nsm / nret));
     cudaError_t e = cudaFuncSetAttribute(spd_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     spd_inverse_kernel<<<dim3(nret, split), kNt, smem, st>>>(d_a, d_ainv, n, stride, d_status);

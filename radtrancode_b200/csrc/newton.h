@@ -46,8 +46,8 @@ cudaError_t launch_newton_step(const NewtonDev* d_ret, int nret, int hessian, in
 // phi (REAL, as the reference function) and chisq per retrieval
 cudaError_t launch_phi(const PhiDev* d_ret, int nret, float* d_phi, float* d_chisq, cudaStream_t st);
 // Sa^-1 from Sa (FP64 Cholesky inverse, dinvertm.f jmod=2) for nret
-// matrices [n][n] at a[r*stride], written to ainv[r*stride]
-cudaError_t launch_spd_inverse(const double* d_a, double* d_ainv, int n, int64_t stride, int nret,
+// matrices [n][n] at a[r*stride], written to ainv[r*stride], on a device of nsm SMs
+cudaError_t launch_spd_inverse(const double* d_a, double* d_ainv, int n, int64_t stride, int nret, int nsm,
                                unsigned* d_status, cudaStream_t st);
 
 }  // namespace rtb

@@ -692,7 +692,7 @@ struct Engine {
             CUDA_TRY(c, cudaMemcpyAsync(Yb(*s), s->y.data(), (size_t)s->ny * 4, cudaMemcpyHostToDevice, st));
             CUDA_TRY(c, cudaMemcpyAsync(Sei(*s), s->sei.data(), (size_t)s->ny * 8, cudaMemcpyHostToDevice, st));
             CUDA_TRY(c, cudaMemcpyAsync(Sa(*s), s->sa.data(), (size_t)s->nx * s->nx * 8, cudaMemcpyHostToDevice, st));
-            CUDA_TRY(c, launch_spd_inverse(Sa(*s), Sai(*s), s->nx, 0, 1, nullptr, st));
+            CUDA_TRY(c, launch_spd_inverse(Sa(*s), Sai(*s), s->nx, 0, 1, c->nsm, nullptr, st));
             active.push_back(s);
         }
         CUDA_TRY(c, cudaStreamSynchronize(st));   // host copies of y/sei/sa stay alive until here
@@ -1080,7 +1080,7 @@ int rtb_spd_inverse_batch(rtb_context* c, int nret, int n, const double* a, doub
     double* D = (double*)c->d_nt64.p;
     CUDA_TRY(c, cudaMemcpyAsync(D, a, nn * nret * 8, cudaMemcpyHostToDevice, st));
     unsigned* status = (unsigned*)c->d_ntsmall.p;
-    CUDA_TRY(c, launch_spd_inverse(D, D + nn * nret, n, (int64_t)nn, nret, status, st));
+    CUDA_TRY(c, launch_spd_inverse(D, D + nn * nret, n, (int64_t)nn, nret, c->nsm, status, st));
     CUDA_TRY(c, cudaMemcpyAsync(ainv, D + nn * nret, nn * nret * 8, cudaMemcpyDeviceToHost, st));
     std::vector<unsigned> sts(nret);
     CUDA_TRY(c, cudaMemcpyAsync(sts.data(), status, 4 * (size_t)nret, cudaMemcpyDeviceToHost, st));
