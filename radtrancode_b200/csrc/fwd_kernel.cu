@@ -637,8 +637,10 @@ __device__ __forceinline__ void cluster_sync() {
 // item worked on at once -- the tile shape the autotuner chooses.  CL = 2: two CTAs
 // of a cluster share an item's layers (the wide tile: B.cluster of them).  The
 // residency bound keeps 24 warps per SM at 80 registers: the passes wait on
-// shuffles and fixed-latency chains, and 16 warps at 128 registers took 4.28 ms
-// where 24 take 4.04 ms (120 layers, 4 absorbers, 2000 wavenumbers).  NGC > 0:
+// shuffles and fixed-latency chains, and 16 warps at 128 registers take 3.83 ms
+// where 24 take 3.27 ms (120 layers, 20-point tables, 4 absorbers, 2000
+// wavenumbers; 60 layers, 10-point tables, 4 absorbers, 1400 wavenumbers 0.78 and
+// 0.71 ms, though 73 layers, 3 absorbers, 515 wavenumbers 0.26 and 0.27).  NGC > 0:
 // NG as a compile-time constant (the overlap's sizes, offsets and loop bounds
 // fold); otherwise NG is read at run time, and -4 or -8 sort the elements of a
 // pass in that many registers per lane, 0 by merging rows
@@ -1058,11 +1060,13 @@ RTB_FWD_PARTS(RTB_FWD_PART_DECL)
 namespace {
 // the instance of a part for an NG: tiles of 2 and 4 warps, and NG = 20 as a
 // constant, exist for the usual options only (one temperature grid, no extended
-// options).  Up to 256 elements a pass are
-// sorted in registers, more are merged in shared memory: one spectrum of
-// 16-point tables (80 layers, 150 wavenumbers, 2 absorbers, a block an item) takes
-// 0.22 ms by the first and 0.27 ms by the second, one of 20-point tables (120
-// layers, 2000 wavenumbers, 4 absorbers) 3.68 and 3.45 ms.
+// options).  Up to 256 elements a pass are sorted in registers, more are merged in
+// shared memory.  By the first and the second: 16-point tables, 80 layers, 2
+// absorbers, 515 wavenumbers 0.33 and 0.37 ms; 10-point tables, 73 layers, 3
+// absorbers, 515 wavenumbers 0.27 and 0.30 ms; 20-point tables, 120 layers, 4
+// absorbers, 2000 wavenumbers 3.69 and 3.27 ms.  With TEMP2 tables and the extended
+// options (80 layers, 3 absorbers, 1500 wavenumbers) 1.24-1.26 and 1.32-1.36 ms at
+// 16 points, 1.23-1.27 and 1.17-1.23 ms at 20.
 constexpr int kNgConst = 20;
 template <bool t2, bool ext, int WARPS, int CL = 1>
 FwdKern fwd_by_ng(int ng) {

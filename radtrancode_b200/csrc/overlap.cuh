@@ -7,13 +7,13 @@
 // in order when B is monotone, in shared memory.  The cumulative weights come
 // from a warp scan, and lane b then walks bin b in the sorted order.
 //
-// What bounds it: instruction issue (2.5 of 4 per cycle and SM with 24 warps) and
+// What bounds it: instruction issue (2.6 of 4 per cycle and SM with 24 warps) and
 // the latency of shared memory and shuffles.  120 layers, 4 absorbers, 2000
 // wavenumbers (720000 passes of 400 keys, a third of them with rows already in
-// order): the forward kernel takes 3.20 ms, 3217 warp instructions a pass.  With
+// order): the forward kernel takes 3.27 ms, 3265 warp instructions a pass.  With
 // the merge on 64-bit words of key and element, and weights and columns in
 // shared-memory tables, it took 5.45 ms (4575 instructions and 585 bank
-// conflicts a pass); with the 400 words sorted in 16 registers a lane 3.68 ms.
+// conflicts a pass); with the 400 words sorted in 16 registers a lane it takes 3.69 ms.
 #pragma once
 #include <stdint.h>
 
@@ -259,7 +259,7 @@ __host__ __device__ constexpr int pass_chunk(int ng) { return (ng * ng + 31) / 3
 // gd and rec each hold NG rows of NG + 1 words, and gd the sequential walk's kMaxCols
 // rows of 32: up to NG 9 those are the most.  Rows of NG words, and rankk's arrays at
 // offsets by NG, would need no more than the elements, but the passes' instances lose
-// by it: 10-point tables, 73 layers, 3 absorbers, 515 wavenumbers take 292 us with
+// by it: 10-point tables, 73 layers, 3 absorbers, 515 wavenumbers took 292 us with
 // them, 276 so.
 __host__ __device__ constexpr int pass_gd_bytes(int ng) {
     const int pref = 8 * 32 * pass_chunk(ng), rows = (4 * ng * (ng + 1) + 15) & ~15, cols = 4 * 32 * kMaxCols;
